@@ -60,7 +60,8 @@ def _stale(obj: str, src: str) -> bool:
 # several instructions fewer each; the form's bar is 1e-5 relative L2)
 _FP32_FAST = ["-prec-div=false", "-prec-sqrt=false"]
 FILE_FLAGS = {"cb_geometry.cu": ["-fmad=false"], "cb_batch_2d_f32.cu": _FP32_FAST, "cb_batch_3d_f32.cu": _FP32_FAST,
-              "cb_inst_2d_f32.cu": _FP32_FAST, "cb_inst_3d_f32.cu": _FP32_FAST}
+              "cb_inst_2d_f32.cu": _FP32_FAST, "cb_inst_3d_f32.cu": _FP32_FAST,
+              "cb_march_f32.cu": _FP32_FAST}
 
 
 def _compile(src: str, verbose: bool) -> tuple[str, str]:

@@ -47,8 +47,9 @@ def nstate(dim: int) -> int:
 def viscous_fused(dim: int, N: int) -> bool:
     """Whether the viscous solver of (dim, N) runs the two fused passes per
     stage (element groups of at most two nodes per thread of a 256-thread
-    block: every 2-D order, 3-D up to N = 7) and so takes state offsets; other
-    orders run the reference's unfused pass sequence."""
+    block: every 2-D order, 3-D up to N = 7) and so takes state offsets, ghosts
+    and stage calls; the other orders run fused passes too (on meshes that are
+    not conforming, the reference's unfused pass sequence) but take none."""
     return dim == 2 or (N + 1) ** 3 <= 512
 
 
@@ -437,7 +438,8 @@ class LSRK:
         check(_lib.lib().cb_solver_status_async(self._h, C.c_void_p(host.data_ptr())))
 
     def set_kernel(self, kernel: int) -> None:
-        """Stage kernel: 0 = the shape's default, 1 = the CUDA-core stages,
+        """Stage kernel: 0 = the shape's default (viscous 3-D: the grid-line
+        passes), 1 = the CUDA-core stages (viscous: the pipelined passes),
         2 = the tensor-core (DMMA) stage of the inviscid 3-D N=7 form, 3 = the
         unpipelined grouped stages (for the fused viscous form: the grouped
         passes instead of the pipelined ones), 4 = the lean pipelined stage

@@ -2,6 +2,7 @@
 // Included once per (dim, precision) translation unit; see cb_inst.cuh.
 #pragma once
 #include "cb_dg.cuh"
+#include "cb_march.h"
 
 namespace cb {
 
@@ -806,6 +807,13 @@ struct Launch {
   // Whether the lean pipelined stage is built for this shape, and whether it
   // is the shape's default (where the tensor-core stage is not).
   static constexpr bool LEAN_OK = Lean<DIM, Nq, T>::OK;
+  // Whether the unpipelined choice (3) and the default are the column march
+  // (cb_march.cuh) instead of the grouped stage: where the all-at-once plan
+  // leaves one block per SM (B200, one mesh of 5.8-6.5 M nodes, ms per step:
+  // N=10 FP64 4.28 -> 3.35, FP32 1.92 -> 1.61; N=9 FP64 2.96 -> 2.72).  Below,
+  // the other stages are the faster ones (N=9 FP32 grouped 1.36, march 1.51;
+  // N=4 FP32 1.21, 1.24; N=7 FP64 tensor-core 1.75, march 2.34).
+  static constexpr bool MARCH = DIM == 3 && (Nq >= 11 || (Nq == 10 && sizeof(T) == 8));
   // Default stage kernel per shape, from B200 timings of one mesh (ms per
   // step, warped 3-D cubes of 7-17 M nodes; pipelined CUDA-core / grouped /
   // lean): FP64 N=3 3.66 / 3.34 / 2.76, N=4 4.95 / 4.20 / 3.78, N=5 2.37 /
@@ -817,7 +825,8 @@ struct Launch {
   // first figure is the grouped stage as well).  3-D N=7 runs the
   // tensor-core stage in both precisions.
   static constexpr int DEFAULT_KERNEL =
-      MMA_DEFAULT ? 2
+      MARCH         ? 3
+      : MMA_DEFAULT ? 2
       : DIM == 3 && sizeof(T) == 8 && LEAN_OK && (Nq == 4 || Nq == 5 || Nq == 9) ? 4
       : DIM == 3 && sizeof(T) == 4 && Nq >= 4 && Nq <= 10 ? 3
       : 1;
@@ -858,6 +867,14 @@ struct Launch {
     constexpr bool pipe_ok = Pipe<DIM, Nq, T>::OK;
     const bool aligned = ((reinterpret_cast<uintptr_t>(Qin) | reinterpret_cast<uintptr_t>(vgeo)) & 15) == 0;
     const bool aligned2 = aligned && ((reinterpret_cast<uintptr_t>(rhs) | reinterpret_cast<uintptr_t>(sgeo)) & 15) == 0;
+    if (ebeg < 0 || ebeg > nelem) return cudaErrorInvalidValue;
+    if constexpr (MARCH) {
+      if (!probe && (kernel == 0 || (kernel == 3 && !ebeg))) {
+        MarchArgs<T> a{Qin, Qout, rhs, vgeo, sgeo, nbr, D, nullptr, ebeg, nelem, {}, rka, rkbdt, status};
+        for (int s = 0; s < NS; ++s) a.qref.v[s] = qref.v[s];
+        return march_stage<T>(Nq, false, a, p, st);
+      }
+    }
     // the shape's default; the grouped stage takes no element range and no
     // test hook: those calls take the pipelined stage, or the lean one where
     // the pipelined plan does not fit shared memory (3-D N=9 FP64, N=10 FP32)
@@ -868,7 +885,6 @@ struct Launch {
     if (kernel == 2 && !(MMA_OK && aligned2)) return cudaErrorNotSupported;
     if (kernel == 4 && !LEAN_OK) return cudaErrorNotSupported;
     if (kernel == 4 && !aligned2) kernel = 1;  // bulk copies need 16-byte aligned slabs
-    if (ebeg < 0 || ebeg > nelem) return cudaErrorInvalidValue;
     const int64_t groups = (nelem - ebeg + C::EPB - 1) / C::EPB;
     if (groups == 0) return cudaSuccess;
     if constexpr (MMA_OK) {

@@ -1,0 +1,2 @@
+#include "cb_march.cuh"
+CB_MARCH_DEFINE(double)

@@ -52,11 +52,12 @@ struct Ops {
   cudaError_t (*update_gradQ)(T *, const T *, const T *, int64_t, int, cudaStream_t);
   cudaError_t (*cons_sums)(const T *, const T *, int64_t, int, const Offs<double, 5> &, double *, int,
                            cudaStream_t);
-  // fused viscous passes over one mesh (pass 0: gradient, 1: stage + update);
-  // nullptr for orders whose groups would need more than two nodes per thread
-  // pass 0 (gradient) or 1 (stage) of the fused viscous form; the last
-  // argument is the solver's kernel choice (3: the grouped stage pass)
+  // fused viscous passes over one mesh: pass 0 (gradient) or 1 (stage +
+  // update); the last argument is the solver's kernel choice
   cudaError_t (*ns_pass)(int, const BDesc<T> &, T *, int64_t, const PhysT<T> &, T, T, cudaStream_t, int);
+  // whether the viscous form of this order has stage calls, ghosts and state
+  // offsets (every 2-D order, 3-D N <= 7)
+  bool ns_stage_form;
 };
 
 // Defined in cb_inst_<dim>d_<prec>.cu; nullptr when N is outside 1..MAXN.

@@ -6,11 +6,11 @@
 // and a solver-owned twin.  Two steps (ten stages) return to the caller's
 // buffer and are captured as one CUDA graph; an odd final step is launched
 // directly and copied back.
-// Viscous (LDG Navier–Stokes) form: for orders whose element groups fit two
-// nodes per thread, two fused passes per stage (gradient, then inviscid +
-// viscous residual and update) that ping-pong like the inviscid form; above
-// that, the reference sequence of passes per stage (volume, face, gradient,
-// divergence, update) on a single buffer, captured one step per graph.
+// Viscous (LDG Navier–Stokes) form: two fused passes per stage (gradient, then
+// inviscid + viscous residual and update) that ping-pong like the inviscid
+// form.  3-D N >= 8 accepts any vmaps: where they do not describe a conforming
+// mesh, it runs the reference sequence of passes per stage (volume, face,
+// gradient, divergence, update) on a single buffer, captured one step per graph.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -50,6 +50,7 @@ struct cb_solver {
   int64_t nghost = 0;  // ghost elements after the nelem own ones in Q and the twin
   int cur = 0;         // stage API: the current state is in Q (0) or in the twin (1)
   int kernel = 0;      // stage kernel choice (cb_solver_set_kernel)
+  bool unfused = false;  // viscous form by the reference's sequence of passes
   int64_t nsplit = -1;  // elements 0 .. nsplit - 1 read no ghost (cb_solver_set_split); -1: not set
 };
 
@@ -66,9 +67,14 @@ const Ops<T> *ops(const cb_solver *s) {
   return s->dim == 2 ? get_ops<2, T>(s->N) : get_ops<3, T>(s->N);
 }
 // viscous form through the two fused passes
-bool fused_visc(const cb_solver *s) {
-  return s->phys.visc > 0 && (s->prec == 64 ? ops<double>(s)->ns_pass != nullptr : ops<float>(s)->ns_pass != nullptr);
+bool fused_visc(const cb_solver *s) { return s->phys.visc > 0 && !s->unfused; }
+// viscous form with stage calls, ghosts and state offsets
+bool ns_stage_form(const cb_solver *s) {
+  return s->phys.visc > 0 && (s->prec == 64 ? ops<double>(s)->ns_stage_form : ops<float>(s)->ns_stage_form);
 }
+// where the fused viscous passes raise the status: the orders without a stage
+// form do not report a non-finite state
+unsigned *visc_status(const cb_solver *s) { return ns_stage_form(s) ? s->status : s->status + 1; }
 // the state ping-pongs between Q and Qalt (two steps per graph)
 bool pingpong(const cb_solver *s) { return s->phys.visc <= 0 || fused_visc(s); }
 
@@ -87,7 +93,7 @@ cudaError_t enqueue_step(cb_solver *s, double dt, bool from_user) {
     I.sgeo = sg;
     I.D = D;
     I.nbr = s->nbr;
-    I.status = s->status;
+    I.status = visc_status(s);
     I.dt = dt;
     for (int k = 0; k < 5; ++k) I.qref[k] = T(s->qref[k]);
     for (int st = 0; st < 5 && e == cudaSuccess; ++st) {
@@ -196,7 +202,7 @@ cudaError_t enqueue_pass(cb_solver *s, int st, double dt, int pass) {
     I.sgeo = (const T *)s->sgeo;
     I.D = (const T *)s->D;
     I.nbr = s->nbr;
-    I.status = s->status;
+    I.status = visc_status(s);
     I.dt = dt;
     for (int k = 0; k < 5; ++k) I.qref[k] = T(s->qref[k]);
     return pass == 0 ? o->ns_pass(0, I, (T *)s->gradQ, s->nelem, p, T(0), T(0), s->stream, s->kernel)
@@ -210,13 +216,17 @@ cudaError_t enqueue_pass(cb_solver *s, int st, double dt, int pass) {
                     p, q5, T(RKA[(st + 1) % 5]), T(RKB[st] * dt), s->status, s->stream, 0, s->kernel, 0);
 }
 
+// The column-march passes (3-D) keep the gradient as records of 12 values per
+// node (cb_march.cuh), the other passes as (Np, nstate, dim, nelem).
+bool grad_records(const cb_solver *s) { return fused_visc(s) && s->dim == 3 && (s->kernel == 0 || !ns_stage_form(s)); }
+
 // Copy whole elements: gather `n` elements listed in `idx` (device int64) of
-// `src` into the contiguous `dst`.
+// `src` (ew values each) into `dst`, one every `dw` values.
 template <typename T>
 __global__ void k_pack(const T *__restrict__ src, const int64_t *__restrict__ idx, int64_t n, int64_t ew,
-                       T *__restrict__ dst) {
+                       int64_t dw, T *__restrict__ dst) {
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n * ew; t += (int64_t)gridDim.x * blockDim.x)
-    dst[t] = src[idx[t / ew] * ew + t % ew];
+    dst[t / ew * dw + t % ew] = src[idx[t / ew] * ew + t % ew];
 }
 
 // Face traces of a partitioned solve.  Entry i of `codes` is (element << 3) |
@@ -224,10 +234,11 @@ __global__ void k_pack(const T *__restrict__ src, const int64_t *__restrict__ id
 // state's fields, or state field x direction for the gradient), each
 // component at element offset Np·c.  Pack reads own elements (0 .. nown - 1)
 // into buf[(i·W + c)·Nfp + fn]; unpack writes ghost slots (element nown + g
-// for code g << 3 | face).  An entry out of range is skipped and raises
-// ST_MESH.
+// for code g << 3 | face).  rec: the gradient as records (component c is
+// direction c / 5 of field c % 5; the density gradient is not kept, its
+// entries are 0).  An entry out of range is skipped and raises ST_MESH.
 template <int DIM, typename T>
-__global__ void k_faces(bool pack, T *__restrict__ arr, const int64_t *__restrict__ codes, int64_t n, int Nq,
+__global__ void k_faces(bool pack, bool rec, T *__restrict__ arr, const int64_t *__restrict__ codes, int64_t n, int Nq,
                         int W, int64_t nown, int64_t nghost, T *__restrict__ buf, unsigned *status) {
   const int Nfp = DIM == 2 ? Nq : Nq * Nq, Np = Nfp * Nq;
   const int64_t per = (int64_t)W * Nfp;
@@ -241,7 +252,12 @@ __global__ void k_faces(bool pack, T *__restrict__ arr, const int64_t *__restric
       continue;
     }
     const int64_t el = pack ? e : nown + e;
-    T *a = arr + face_node_rt<DIM>(Nq, f, fn) + (int64_t)Np * (c + (int64_t)W * el);
+    const int64_t node = face_node_rt<DIM>(Nq, f, fn);
+    if (rec && c % 5 == 3) {
+      if (pack) buf[t] = T(0);
+      continue;
+    }
+    T *a = rec ? arr + 12 * (node + Np * el) + 4 * (c / 5) + (c % 5 == 4 ? 3 : c % 5) : arr + node + (int64_t)Np * (c + (int64_t)W * el);
     if (pack) buf[t] = *a;
     else *a = buf[t];
   }
@@ -252,12 +268,13 @@ cudaError_t launch_faces(const cb_solver *s, bool pack, int what, const int64_t 
   const int Nq = s->N + 1, Nfp = s->dim == 2 ? Nq : Nq * Nq;
   const int W = (s->dim == 2 ? 4 : 5) * (what ? s->dim : 1);
   T *arr = (T *)(what ? s->gradQ : (s->cur ? s->Qalt : s->Q));
+  const bool rec = what && grad_records(s);
   const int64_t total = n * W * Nfp;
   const int grid = (int)std::min<int64_t>((total + 255) / 256, 148 * 16);
   if (s->dim == 2)
-    k_faces<2, T><<<grid, 256, 0, s->stream>>>(pack, arr, codes, n, Nq, W, s->nelem, s->nghost, (T *)buf, s->status);
+    k_faces<2, T><<<grid, 256, 0, s->stream>>>(pack, rec, arr, codes, n, Nq, W, s->nelem, s->nghost, (T *)buf, s->status);
   else
-    k_faces<3, T><<<grid, 256, 0, s->stream>>>(pack, arr, codes, n, Nq, W, s->nelem, s->nghost, (T *)buf, s->status);
+    k_faces<3, T><<<grid, 256, 0, s->stream>>>(pack, rec, arr, codes, n, Nq, W, s->nelem, s->nghost, (T *)buf, s->status);
   return cudaGetLastError();
 }
 
@@ -355,7 +372,8 @@ int cb_solver_create_ghosted(cb_solver **out, int dim, int N, int precision, int
 int cb_solver_stage_pass(cb_solver *s, int stage, double dt, int pass, void **next_in) {
   if (!s || stage < 0 || stage > 4 || pass < 0 || pass > 1)
     return solver_fail(CB_ERR_ARG, "cb_solver_stage_pass: bad arguments");
-  if (!pingpong(s)) return solver_fail(CB_ERR_UNSUPPORTED, "cb_solver_stage: this viscous order has no stage form");
+  if (s->phys.visc > 0 && !ns_stage_form(s))
+    return solver_fail(CB_ERR_UNSUPPORTED, "cb_solver_stage: this viscous order has no stage form");
   const cudaError_t e =
       s->prec == 64 ? enqueue_pass<double>(s, stage, dt, pass) : enqueue_pass<float>(s, stage, dt, pass);
   if (e != cudaSuccess) return solver_fail(CB_ERR_CUDA, "cb_solver_stage: %s", cudaGetErrorString(e));
@@ -386,13 +404,15 @@ int cb_solver_pack(cb_solver *s, int what, const int64_t *elems, int64_t n, void
     return solver_fail(CB_ERR_ARG, "cb_solver_pack: bad arguments");
   if (!n) return CB_OK;
   const int Nq = s->N + 1;
-  const int64_t ew = (s->dim == 2 ? (int64_t)Nq * Nq * 4 : (int64_t)Nq * Nq * Nq * 5) * (what ? s->dim : 1);
+  const int64_t Np = s->dim == 2 ? (int64_t)Nq * Nq : (int64_t)Nq * Nq * Nq;
+  const int64_t dw = Np * (s->dim == 2 ? 4 : 5) * (what ? s->dim : 1);
+  const int64_t ew = what && grad_records(s) ? 12 * Np : dw;
   const int grid = (int)std::min<int64_t>((n * ew + 255) / 256, 148 * 16);
   const void *src = what ? s->gradQ : (s->cur ? s->Qalt : s->Q);
   if (s->prec == 64)
-    k_pack<double><<<grid, 256, 0, s->stream>>>((const double *)src, elems, n, ew, (double *)buf);
+    k_pack<double><<<grid, 256, 0, s->stream>>>((const double *)src, elems, n, ew, dw, (double *)buf);
   else
-    k_pack<float><<<grid, 256, 0, s->stream>>>((const float *)src, elems, n, ew, (float *)buf);
+    k_pack<float><<<grid, 256, 0, s->stream>>>((const float *)src, elems, n, ew, dw, (float *)buf);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? CB_OK : solver_fail(CB_ERR_CUDA, "cb_solver_pack: %s", cudaGetErrorString(e));
 }
@@ -403,9 +423,10 @@ int cb_solver_unpack(cb_solver *s, int what, const void *buf, int64_t first, int
   if (first < 0 || n < 0 || first + n > s->nghost || (n && !buf))
     return solver_fail(CB_ERR_ARG, "cb_solver_unpack: ghost range outside 0..%lld", (long long)s->nghost);
   if (!n) return CB_OK;
-  const size_t ew = state_bytes(s) / (size_t)s->nelem * (what ? s->dim : 1);
+  const size_t sw = state_bytes(s) / (size_t)s->nelem * (what ? s->dim : 1);  // bytes per element in buf
+  const size_t ew = what && grad_records(s) ? sw / 15 * 12 : sw;
   char *dst = (char *)(what ? s->gradQ : (s->cur ? s->Qalt : s->Q)) + ew * (size_t)(s->nelem + first);
-  const cudaError_t e = cudaMemcpyAsync(dst, buf, ew * (size_t)n, cudaMemcpyDeviceToDevice, s->stream);
+  const cudaError_t e = cudaMemcpy2DAsync(dst, ew, buf, sw, ew, (size_t)n, cudaMemcpyDeviceToDevice, s->stream);
   return e == cudaSuccess ? CB_OK : solver_fail(CB_ERR_CUDA, "cb_solver_unpack: %s", cudaGetErrorString(e));
 }
 
@@ -454,12 +475,12 @@ int solver_create(cb_solver **out, int dim, int N, int precision, int64_t nelem,
     if ((e = cudaStreamCreate(&s->stream)) != cudaSuccess) return bail(CB_ERR_CUDA, "stream");
     s->own_stream = true;
   }
-  if ((e = cudaMalloc(&s->status, sizeof(unsigned))) != cudaSuccess) return bail(CB_ERR_NOMEM, "status");
-  cudaMemsetAsync(s->status, 0, sizeof(unsigned), s->stream);
+  if ((e = cudaMalloc(&s->status, 2 * sizeof(unsigned))) != cudaSuccess) return bail(CB_ERR_NOMEM, "status");
+  cudaMemsetAsync(s->status, 0, 2 * sizeof(unsigned), s->stream);
   s->part_blocks = 296;
   if ((e = cudaMalloc(&s->part, sizeof(double) * 4 * ns * s->part_blocks)) != cudaSuccess)
     return bail(CB_ERR_NOMEM, "partials");
-  if (phys->visc > 0 && nghost > 0 && !fused_visc(s)) {
+  if (phys->visc > 0 && nghost > 0 && !ns_stage_form(s)) {
     cb_solver_destroy(s);
     return solver_fail(CB_ERR_UNSUPPORTED, "cb_solver_create_ghosted: this viscous order has no stage form");
   }
@@ -467,10 +488,6 @@ int solver_create(cb_solver **out, int dim, int N, int precision, int64_t nelem,
     const size_t gbytes = w * (size_t)Np * ns * dim * (nelem + nghost);
     if ((e = cudaMalloc(&s->gradQ, gbytes)) != cudaSuccess) return bail(CB_ERR_NOMEM, "gradQ");
     cudaMemsetAsync(s->gradQ, 0, gbytes, s->stream);
-    if (!fused_visc(s)) {
-      if ((e = cudaMalloc(&s->rhs_gradQ, gbytes)) != cudaSuccess) return bail(CB_ERR_NOMEM, "rhs_gradQ");
-      cudaMemsetAsync(s->rhs_gradQ, 0, gbytes, s->stream);
-    }
   }
   if (pingpong(s)) {
     if ((e = cudaMalloc(&s->Qalt, w * (size_t)Np * ns * (nelem + nghost))) != cudaSuccess)
@@ -508,6 +525,18 @@ int solver_create(cb_solver **out, int dim, int N, int precision, int64_t nelem,
   if ((e = cudaMemcpyAsync(&h, s->status, sizeof h, cudaMemcpyDeviceToHost, s->stream)) != cudaSuccess ||
       (e = cudaStreamSynchronize(s->stream)) != cudaSuccess)
     return bail(CB_ERR_CUDA, "setup");
+  if (h && phys->visc > 0 && !ns_stage_form(s)) {  // no neighbour table: the reference's sequence of passes
+    s->unfused = true;
+    cudaFree(s->Qalt);
+    cudaFree(s->nbr);
+    s->Qalt = nullptr;
+    s->nbr = nullptr;
+    h = 0;
+    const size_t gbytes = w * (size_t)Np * ns * dim * nelem;
+    if ((e = cudaMalloc(&s->rhs_gradQ, gbytes)) != cudaSuccess) return bail(CB_ERR_NOMEM, "rhs_gradQ");
+    cudaMemsetAsync(s->rhs_gradQ, 0, gbytes, s->stream);
+    cudaMemsetAsync(s->status, 0, 2 * sizeof(unsigned), s->stream);
+  }
   if (h & ST_BC) {
     cb_solver_destroy(s);
     return solver_fail(CB_ERR_BC, "invalid boundary condition code (only 0 and 1 are defined)");
@@ -594,7 +623,7 @@ int cb_solver_sums(cb_solver *s, double *out_host) {
 
 int cb_solver_set_offset(cb_solver *s, const double *qref) {
   if (!s || !qref) return solver_fail(CB_ERR_ARG, "null argument");
-  if (s->phys.visc > 0 && !fused_visc(s)) {
+  if (s->phys.visc > 0 && !ns_stage_form(s)) {
     for (int k = 0; k < (s->dim == 2 ? 4 : 5); ++k)
       if (qref[k] != 0.0)
         return solver_fail(CB_ERR_UNSUPPORTED, "state offsets: the viscous form of this order has none");

@@ -189,11 +189,13 @@ int cb_solver_status_async(cb_solver *s, unsigned *out_host);
  * stage of the inviscid form (D contraction on the FP64 tensor pipe as 8x8x4
  * DMMA tiles, for FP32 solvers on the FP32 fluxes converted to FP64, the sum
  * rounded once; built for 3-D N=7, CB_ERR_UNSUPPORTED elsewhere), 3 = the
- * unpipelined grouped stages (the inviscid k_stage; for the fused viscous
- * form the grouped passes instead of the pipelined ones), 4 = the lean
+ * unpipelined grouped stages (the inviscid k_stage, the column march at 3-D
+ * N=10 and FP64 N=9; for the fused viscous form the grouped passes), 4 = the lean
  * pipelined stage of the inviscid form (only the state staged in shared
  * memory, the geometry and carry read from L2; bit-identical to 1).  The
- * default is the fastest on B200 for the shape.  All agree with the oracle
+ * default is the fastest on B200 for the shape (viscous 3-D: the grid-line
+ * passes, with 1 the pipelined ones up to N=7; 3-D N >= 8 has only the
+ * grid-line passes).  All agree with the oracle
  * to round-off; changing it re-captures the step graph at the next run.
  * cb_solver_get_kernel reports the kernel the solver runs (1 to 4). */
 int cb_solver_set_kernel(cb_solver *s, int kernel);
