@@ -121,16 +121,13 @@ __device__ __forceinline__ void stage_group(const BDesc<T> &I, int64_t e0, int n
       const T gc = p.grav != T(0) ? vg[n + Np * GC] : T(0);
       const T ri = T(1) / q[IR];
       const T P = pressure_ri<DIM, T>(q, ri, gc, p);
-      T f[NS][DIM];
-      euler_flux_ri<DIM, T>(q, ri, P, f);
 #pragma unroll
-      for (int r = 0; r < DIM; ++r)
+      for (int r = 0; r < DIM; ++r) {
+        T f[NS];
+        contravariant_flux<DIM, T>(q, ri, P, MJ, met[r], f);
 #pragma unroll
-        for (int s = 0; s < NS; ++s) {
-          T a = met[r][0] * f[s][0] + met[r][1] * f[s][1];
-          if (DIM == 3) a = a + met[r][2] * f[s][2];
-          sF[(r * NS + s) * SP + el * Np + n] = MJ * a;
-        }
+        for (int s = 0; s < NS; ++s) sF[(r * NS + s) * SP + el * Np + n] = f[s];
+      }
       R[u][DIM - 1] -= MJ * q[IR] * p.grav;
     }
   }

@@ -196,7 +196,7 @@ k_stage(const T *__restrict__ Qin, T *__restrict__ Qout, T *__restrict__ rhs,
         int64_t nelem, PhysT<T> p, Offs<T, Lay<DIM>::NS> qref, T rka, T rkbdt,
         unsigned *status) {
   using C = Cfg<DIM, Nq>;
-  constexpr int NS = Lay<DIM>::NS, NVG = Lay<DIM>::NVG, NSG = Lay<DIM>::NSG;
+  constexpr int NS = Lay<DIM>::NS, NVG = Lay<DIM>::NVG, NSG = Lay<DIM>::NSG, IR = Lay<DIM>::IR;
   constexpr int Np = C::Np, Nfp = C::Nfp, NF = C::NFACE, SP = C::SLOTS;
   constexpr int FS = C::EPB * Nfp, MJI = DIM * DIM + 1;
   constexpr int GC = DIM * DIM + 2 + DIM - 1;
@@ -222,7 +222,7 @@ k_stage(const T *__restrict__ Qin, T *__restrict__ Qout, T *__restrict__ rhs,
         q[s] = d + qref.v[s];
         R[u][s] = rhs[n + Np * (s + NS * e)];
       }
-      pointwise_euler<DIM, Nq, C::EPB, T>(q, vgeo + (int64_t)Np * NVG * e, n, el, sF, p, R[u]);
+      pointwise_euler_n<DIM, Nq, C::EPB, T>(q, vgeo + (int64_t)Np * NVG * e, n, el, sF, p, R[u]);
     }
   }
   __syncthreads();
@@ -253,22 +253,25 @@ k_stage(const T *__restrict__ Qin, T *__restrict__ Qout, T *__restrict__ rhs,
 #pragma unroll
     for (int s = 0; s < NS; ++s) qM[s] = sQ[s * SP + el * Np + vM] + qref.v[s];
     const T gM = p.grav != T(0) ? vgeo[vM + Np * (GC + NVG * e)] : T(0);
-    const T PM = pressure<DIM, T>(qM, gM, p);
+    const T riM = T(1) / qM[IR];
+    const T PM = pressure_ri<DIM, T>(qM, riM, gM, p);
     const int32_t nb = nbr[f + NF * e];
-    T PP;
+    T PP, riP;
     if (nb >= 0) {
       const int64_t e2 = nb >> 3;
       const int vP = face_node<DIM, Nq>(nb & 7, fn);
 #pragma unroll
       for (int s = 0; s < NS; ++s) qP[s] = Qin[vP + Np * (s + NS * e2)] + qref.v[s];
       const T gP = p.grav != T(0) ? vgeo[vP + Np * (GC + NVG * e2)] : T(0);
-      PP = pressure<DIM, T>(qP, gP, p);
+      riP = T(1) / qP[IR];
+      PP = pressure_ri<DIM, T>(qP, riP, gP, p);
     } else {
       wall_state<DIM, T>(qM, nrm, qP);
+      riP = riM;
       PP = PM;
     }
     T out[NS];
-    rusanov<DIM, T>(qM, PM, qP, PP, nrm, p, out);
+    rusanov_n<DIM, T>(qM, riM, PM, qP, riP, PP, nrm, p, out);
 #pragma unroll
     for (int s = 0; s < NS; ++s) FF[(f * NS + s) * FS + el * Nfp + fn] = sMJ * out[s];
   }

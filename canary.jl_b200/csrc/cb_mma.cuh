@@ -98,7 +98,10 @@ struct PipeMT {
   // SM if the registers fit 85 per thread (measured at 32^3: 0.566 ms per
   // stage; four blocks at 64 registers spill and take 0.637 ms)
   // (FP32 with the prefetch one group ahead: 0.567 ms, the same)
-  static constexpr int MINB = sizeof(T) == 8 ? 2 : 3, PFD = -1;
+  // PFD = -2: one group ahead, at the middle of the iteration (FP32 with its
+  // half-size plan: 2.54 ms per step at 32^3 against 2.60; FP64, whose blocks
+  // then hold too much of L2: 5.21 against 4.86)
+  static constexpr int MINB = sizeof(T) == 8 ? 2 : 3, PFD = sizeof(T) == 8 ? -1 : -2;
   // whether this stage is the default of its shape (the faster on B200 at
   // 32^3 hexes: FP64 0.974 ms per stage against 1.17 ms for the CUDA-core
   // stage, FP32 0.719 against 0.744 ms)
@@ -127,8 +130,9 @@ __device__ __forceinline__ int fg_pos(int i, int j) { return j * 8 + (i ^ (((j >
 // MINB: resident blocks per SM the registers are sized for; PFD: how many
 // groups ahead the bulk L2 prefetch of a group's metric, carry and face
 // geometry is issued (0: none, the loads go to HBM directly; -1: for the
-// group itself, at the top of its iteration).
-template <typename Src, int MINB = PipeM::MINB, int PFD = PipeM::PFD>
+// group itself, at the top of its iteration; -2: for the next group, at the
+// middle of an iteration).
+template <typename Src, int MINB = PipeM::MINB, int PFD = PipeMT<typename Src::Real>::PFD>
 __global__ void __launch_bounds__(PipeM::THREADS, MINB)
     k_stage_mma(Src src, PhysT<typename Src::Real> p, typename Src::Real rka) {
   using T = typename Src::Real;  // storage (and, for float, flux and update arithmetic)
@@ -210,7 +214,7 @@ __global__ void __launch_bounds__(PipeM::THREADS, MINB)
     const int64_t e0 = src.e0(it);
     const bool more = src.valid(it + 1);
     if (PFD > 0 && tid == 0 && src.valid(it + PFD)) prefetch_group(it + PFD);
-    if (PFD < 0 && tid == 0) prefetch_group(it);
+    if (tid == 0 && (PFD == -1 || (PFD == -2 && it == 0))) prefetch_group(it);
     if (tid == Src::PUBLISHER) src.prefetch();
     const T *__restrict__ Qin = src.Qin(it);
     const T *__restrict__ vg = src.vgeo(it) + e0 * Np * NVG;
@@ -332,18 +336,17 @@ __global__ void __launch_bounds__(PipeM::THREADS, MINB)
       const T gc = p.grav != T(0) ? vg[n + Np * GC] : T(0);
       const T ri = T(1) / q[IR];
       const T P = pressure_ri<DIM, T>(q, ri, gc, p);
-      T f[NS][DIM];
-      euler_flux_ri<DIM, T>(q, ri, P, f);
       const int pf = fg_pos(2 * t + c, g);
 #pragma unroll
-      for (int r = 0; r < DIM; ++r)
+      for (int r = 0; r < DIM; ++r) {
+        T f[NS];
+        contravariant_flux<DIM, T>(q, ri, P, MJ, mt[r], f);
 #pragma unroll
         for (int s = 0; s < NS; ++s) {
-          T a = mt[r][0] * f[s][0] + mt[r][1] * f[s][1];
-          a = a + mt[r][2] * f[s][2];
           T *dst = r < 2 ? FG + (s * 2 + r) * 64 : HZ + s * PM::HS + w * PM::HP;
-          dst[pf] = MJ * a;
+          dst[pf] = f[s];
         }
+      }
       buoy[c] = MJ * q[IR] * p.grav;
     }
     __syncwarp();
@@ -374,7 +377,10 @@ __global__ void __launch_bounds__(PipeM::THREADS, MINB)
       if constexpr (PM::ASYNC_QP) cp_async_wait<0>();  // this thread's trace copies land before the block leaves
       return;
     }
-    if (tid == 0 && more) issue_S(it + 1);
+    if (tid == 0 && more) {
+      issue_S(it + 1);
+      if (PFD == -2) prefetch_group(it + 1);
+    }
     if ((tid >> 5) == (Src::PUBLISHER >> 5)) src.publish(it);
 
     // ---- zeta products: warp w computes rows (i, j = w), columns k, and

@@ -404,18 +404,14 @@ k_stage_pipe2(Src src, PhysT<T> p, T rka) {
         }
         const T ri = T(1) / q[IR];
         const T P = pressure_ri<DIM, T>(q, ri, gc, p);
-        T f[NS][DIM];
-        euler_flux_ri<DIM, T>(q, ri, P, f);
 #pragma unroll
         for (int r = 0; r < DIM; ++r) {
           const int row = DIM == 2 ? (r == 0 ? j : i) : (r == 0 ? j + Nq * k : (r == 1 ? i + Nq * k : i + Nq * j));
           const int pos = r == 0 ? i : (r == 1 ? j : k);
+          T f[NS];
+          contravariant_flux<DIM, T>(q, ri, P, MJ, met[r], f);
 #pragma unroll
-          for (int s = 0; s < NS; ++s) {
-            T a = met[r][0] * f[s][0] + met[r][1] * f[s][1];
-            if (DIM == 3) a = a + met[r][2] * f[s][2];
-            sF[r * PP::FDIR + ((size_t)(s * EPB + el) * NR + row) * RS + pos] = MJ * a;
-          }
+          for (int s = 0; s < NS; ++s) sF[r * PP::FDIR + ((size_t)(s * EPB + el) * NR + row) * RS + pos] = f[s];
         }
         buoy[u] = MJ * q[IR] * p.grav;
       }
