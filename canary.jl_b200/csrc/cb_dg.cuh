@@ -16,6 +16,39 @@
 
 namespace cb {
 
+// Programmatic launch of the stage kernels.  A solver's stages depend on one
+// another, and on small meshes a stage is shorter than the gap between two
+// launches; the next stage's blocks are therefore launched, initialise their
+// barriers and read what no stage writes while the current stage finishes.
+// grid_wait (all threads, before anything that a stage writes is read or
+// written) returns once the preceding grid is complete and its writes visible;
+// only then is the dependent grid let go, so that no grid starts while the one
+// two before it still reads the buffer which it will read.  The pointers depend
+// on the instruction: loads from them (read-only data to the compiler) cannot be
+// moved above it.  Both instructions do nothing in a plain launch.
+template <typename... P>
+__device__ __forceinline__ void grid_wait(P *&...ptr) {
+  int64_t zero;
+  asm volatile("griddepcontrol.wait;\n\tmov.s64 %0, 0;" : "=l"(zero)::"memory");
+  ((void)(ptr += zero), ...);  // (an offset: the compiler still knows that they point to global memory)
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <typename... K, typename... A>
+inline cudaError_t launch_stage_kernel(void (*kernel)(K...), unsigned grid, int threads, size_t smem, cudaStream_t st,
+                                       const A &...args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3(threads);
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, kernel, K(args)...);
+}
+
 // Mirror of the public cb_phys.
 struct Phys {
   double gamma, R_gas, c_p, c_v, gravity, Pr, lambda, visc;

@@ -190,11 +190,11 @@ __global__ void k_update(T *__restrict__ rhs, const T *__restrict__ rhs_gradQ,
 // ======================================================================
 template <int DIM, int Nq, typename T>
 __global__ void __launch_bounds__(Cfg<DIM, Nq>::THREADS)
-k_stage(const T *__restrict__ Qin, T *__restrict__ Qout, T *__restrict__ rhs,
+k_stage(const T *Qin_, T *Qout_, T *rhs_,
         const T *__restrict__ vgeo, const T *__restrict__ sgeo,
         const int32_t *__restrict__ nbr, const T *__restrict__ D,
         int64_t nelem, PhysT<T> p, Offs<T, Lay<DIM>::NS> qref, T rka, T rkbdt,
-        unsigned *status) {
+        unsigned *status, int64_t ebeg) {
   using C = Cfg<DIM, Nq>;
   constexpr int NS = Lay<DIM>::NS, NVG = Lay<DIM>::NVG, NSG = Lay<DIM>::NSG, IR = Lay<DIM>::IR;
   constexpr int Np = C::Np, Nfp = C::Nfp, NF = C::NFACE, SP = C::SLOTS;
@@ -205,7 +205,11 @@ k_stage(const T *__restrict__ Qin, T *__restrict__ Qout, T *__restrict__ rhs,
   T *sQ = Ds + ((Nq * Nq + 1) & ~1);  // [NS][SP]
   T *sF = sQ + NS * SP;               // [DIM][NS][SP], reused as FF
   load_D(Ds, D, Nq * Nq);
-  const int64_t e0 = (int64_t)blockIdx.x * C::EPB;
+  grid_wait(Qin_, Qout_, rhs_);
+  const T *__restrict__ Qin = Qin_;
+  T *__restrict__ Qout = Qout_;
+  T *__restrict__ rhs = rhs_;
+  const int64_t e0 = ebeg + (int64_t)blockIdx.x * C::EPB;
   T R[C::NPT][NS];
   // ---- pointwise fluxes
 #pragma unroll
@@ -825,13 +829,14 @@ struct Launch {
   // 2.02 / 1.68 / 2.61, N=8 3.08 / 2.61 / 3.44, N=9 2.22 / 1.93 / 2.45 (the
   // FP32 pipelined plans fit fewer blocks per SM than the grouped stage;
   // FP64 N=8, 9 have no pipelined plan that fits shared memory, so their
-  // first figure is the grouped stage as well).  3-D N=7 runs the
-  // tensor-core stage in both precisions.
+  // first figure is the grouped stage as well).  N=2, 6.1 M nodes: FP64 4.30 /
+  // 3.18 / 3.42, FP32 1.83 / 1.33 / 1.64; N=1: FP64 4.52 / 3.30 / 3.90, FP32
+  // 2.87 / 1.36 / 2.43.  3-D N=7 runs the tensor-core stage in both precisions.
   static constexpr int DEFAULT_KERNEL =
       MARCH         ? 3
       : MMA_DEFAULT ? 2
       : DIM == 3 && sizeof(T) == 8 && LEAN_OK && (Nq == 4 || Nq == 5 || Nq == 9) ? 4
-      : DIM == 3 && sizeof(T) == 4 && Nq >= 4 && Nq <= 10 ? 3
+      : DIM == 3 && (Nq <= 3 || (sizeof(T) == 4 && Nq <= 10)) ? 3
       : 1;
   static constexpr bool LEAN_DEFAULT = DEFAULT_KERNEL == 4;
   // Resident blocks per SM of a kernel at `smem` bytes, from the occupancy
@@ -878,12 +883,13 @@ struct Launch {
         return march_stage<T>(Nq, false, a, p, st);
       }
     }
-    // the shape's default; the grouped stage takes no element range and no
-    // test hook: those calls take the pipelined stage, or the lean one where
-    // the pipelined plan does not fit shared memory (3-D N=9 FP64, N=10 FP32)
-    if (kernel == 0 && (probe || ebeg) && (DEFAULT_KERNEL == 1 || DEFAULT_KERNEL == 3))
+    // the shape's default; the grouped stage takes no test hook: that call
+    // takes the pipelined stage, or the lean one where the pipelined plan does
+    // not fit shared memory (3-D N=10 FP32)
+    const bool grouped_default = kernel == 0 && DEFAULT_KERNEL == 3 && !probe;
+    if (kernel == 0 && (probe || ebeg) && !grouped_default && (DEFAULT_KERNEL == 1 || DEFAULT_KERNEL == 3))
       kernel = (Pipe2<DIM, Nq, T>::OK || !LEAN_OK) ? 1 : 4;
-    else if (kernel == 0 && DEFAULT_KERNEL == 3)
+    else if (grouped_default)
       kernel = 3;
     if (kernel == 2 && !(MMA_OK && aligned2)) return cudaErrorNotSupported;
     if (kernel == 4 && !LEAN_OK) return cudaErrorNotSupported;
@@ -901,8 +907,7 @@ struct Launch {
         int64_t g = (int64_t)num_sms() * bps;
         if (g > groups) g = groups;
         const S src{Qin, Qout, rhs, vgeo, sgeo, nbr, D, nelem, qref, rkbdt, status, probe, ebeg};
-        k_stage_mma<S, PM::MINB><<<(int)g, PM::THREADS, PM::smem(), st>>>(src, p, rka);
-        return cudaGetLastError();
+        return launch_stage_kernel(k_stage_mma<S, PM::MINB>, (unsigned)g, PM::THREADS, PM::smem(), st, src, p, rka);
       }
     }
     if constexpr (LEAN_OK) {
@@ -916,8 +921,7 @@ struct Launch {
         int64_t g = (int64_t)num_sms() * bps;
         if (g > groups) g = groups;
         const S src{Qin, Qout, rhs, vgeo, sgeo, nbr, D, nelem, qref, rkbdt, status, probe, ebeg};
-        k_stage_lean<DIM, Nq, T, S><<<(int)g, C::THREADS, PL::smem(), st>>>(src, p, rka);
-        return cudaGetLastError();
+        return launch_stage_kernel(k_stage_lean<DIM, Nq, T, S>, (unsigned)g, C::THREADS, PL::smem(), st, src, p, rka);
       }
     }
     if (Pipe2<DIM, Nq, T>::OK && aligned2 && kernel != 3) {
@@ -931,9 +935,8 @@ struct Launch {
       int64_t g = (int64_t)num_sms() * bps;
       if (g > groups) g = groups;
       const S src{Qin, Qout, rhs, vgeo, sgeo, nbr, D, nelem, qref, rkbdt, status, probe, ebeg};
-      k_stage_pipe2<DIM, Nq, T, S><<<(int)g, C::THREADS, sm, st>>>(src, p, rka);
-      return cudaGetLastError();
-    } else if (probe || ebeg) {
+      return launch_stage_kernel(k_stage_pipe2<DIM, Nq, T, S>, (unsigned)g, C::THREADS, sm, st, src, p, rka);
+    } else if (probe || (ebeg && !grouped_default)) {
       return cudaErrorNotSupported;
     } else if (pipe_ok && aligned && kernel != 3) {
       using PP = Pipe<DIM, Nq, T>;
@@ -949,9 +952,8 @@ struct Launch {
       size_t sm = smem_stage();
       cudaError_t err = prep(k_stage<DIM, Nq, T>, sm);
       if (err != cudaSuccess) return err;
-      k_stage<DIM, Nq, T><<<grid(nelem), C::THREADS, sm, st>>>(Qin, Qout, rhs, vgeo, sgeo, nbr, D,
-                                                                nelem, p, qref, rka, rkbdt, status);
-      return cudaGetLastError();
+      return launch_stage_kernel(k_stage<DIM, Nq, T>, (unsigned)groups, C::THREADS, sm, st, Qin, Qout, rhs, vgeo, sgeo,
+                                 nbr, D, nelem, p, qref, rka, rkbdt, status, ebeg);
     }
   }
   // Whether stage() takes an element range (ebeg > 0) for arrays aligned

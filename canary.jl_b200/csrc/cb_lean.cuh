@@ -89,7 +89,6 @@ k_stage_lean(Src src, PhysT<T> p, T rka) {
     if (L) bulk_g2s(Sq0, base, L, bar);
   };
 
-  src.begin(smem_raw + PP::smem());
   if (tid == 0) {
     mbar_init(bar, 1);
     fence_mbar_init();
@@ -97,6 +96,7 @@ k_stage_lean(Src src, PhysT<T> p, T rka) {
   if constexpr (PP::MV > Nq)
     for (size_t t = tid; t < (size_t)DIM * PP::FDIR; t += C::THREADS)
       if ((int)(t % RS) >= Nq) sF[t] = T(0);
+  src.begin(smem_raw + PP::smem());
   __syncthreads();
   if (tid == 0 && src.valid(0)) issue(0);
 

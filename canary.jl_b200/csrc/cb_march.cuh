@@ -202,6 +202,7 @@ __global__ void __launch_bounds__(March<Nq, T>::THREADS,
   T *DT = reinterpret_cast<T *>(smem_raw + C::OFF_DT), *DZ = reinterpret_cast<T *>(smem_raw + C::OFF_DZ);
   T *PL = reinterpret_cast<T *>(smem_raw + C::OFF_P);
   T *FF = reinterpret_cast<T *>(smem_raw + C::OFF_FF);
+  grid_wait(a.Qin, a.Qout, a.rhs, a.gq);
   const int tid = threadIdx.x, el = tid / N2, ij = tid % N2, i = ij % Nq, j = ij / Nq;
   const int64_t e0 = a.ebeg + (int64_t)blockIdx.x * EPB, e = e0 + el;
   const bool act = el < EPB && e < a.eend;
@@ -468,6 +469,7 @@ __global__ void __launch_bounds__(March<Nq, T>::THREADS, March<Nq, T>::blocks_fo
   using V = typename Vec16<T>::type;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T *DS = reinterpret_cast<T *>(smem_raw), *S = reinterpret_cast<T *>(smem_raw + C::OFF_S);
+  grid_wait(A.Qin, A.gq);
   const int tid = threadIdx.x, el = tid / N2, ab = tid % N2;
   const int64_t e0 = A.ebeg + (int64_t)blockIdx.x * EPB;
   LineCtx<Nq, T> c;
@@ -604,8 +606,7 @@ struct MarchLaunch {
       const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return e;
     }
-    kernel<<<(unsigned)g, M::THREADS, smem, st>>>(a, p);
-    return cudaGetLastError();
+    return launch_stage_kernel(kernel, (unsigned)g, M::THREADS, smem, st, a, p);
   }
   static cudaError_t stage(bool visc, const MarchArgs<T> &a, const PhysT<T> &p, cudaStream_t st) {
     return visc ? launch(k_march_stage<Nq, T, true>, M::smem_stage(), a, p, st)

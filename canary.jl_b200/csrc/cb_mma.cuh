@@ -165,11 +165,11 @@ __global__ void __launch_bounds__(PipeM::THREADS, MINB)
     prefetch_l2(src.sgeo(it) + e * (int64_t)(NSG * Nfp * NF), (uint32_t)PM::SB);
   };
 
-  src.begin(smem_raw + PM::smem());
   if (tid == 0) {
     mbar_init(&barS[0], 1);
     fence_mbar_init();
   }
+  src.begin(smem_raw + PM::smem());
   __syncthreads();
   if (tid == 0 && src.valid(0)) {
     issue_S(0);

@@ -126,7 +126,6 @@ k_ns_stage_pipe(Src src, PhysT<T> p, T rka) {
     rag(Sg0, g, nv * PP::GQB, last, true);
   };
 
-  src.begin(smem_raw + PP::smem());
   if (tid == 0) {
     mbar_init(bar, 1);
     fence_mbar_init();
@@ -134,6 +133,7 @@ k_ns_stage_pipe(Src src, PhysT<T> p, T rka) {
   if constexpr (PP::MV > Nq)
     for (size_t t = tid; t < (size_t)DIM * PP::FDIR; t += C::THREADS)
       if ((int)(t % RS) >= Nq) sF[t] = T(0);
+  src.begin(smem_raw + PP::smem());
   __syncthreads();
   if (tid == 0 && src.valid(0)) issue(0);
 
@@ -484,7 +484,6 @@ k_ns_grad_pipe(Src src, PhysT<T> p, T) {
     if (L) bulk_g2s(Sq0, base, L, bar);
   };
 
-  src.begin(smem_raw + PP::smem());
   if (tid == 0) {
     mbar_init(bar, 1);
     fence_mbar_init();
@@ -492,6 +491,7 @@ k_ns_grad_pipe(Src src, PhysT<T> p, T) {
   if constexpr (PS::MV > Nq)
     for (size_t t = tid; t < (size_t)DIM * PS::FDIR; t += C::THREADS)
       if ((int)(t % RS) >= Nq) sF[t] = T(0);
+  src.begin(smem_raw + PP::smem());
   __syncthreads();
   if (tid == 0 && src.valid(0)) issue(0);
 

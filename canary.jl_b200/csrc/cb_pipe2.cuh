@@ -142,7 +142,7 @@ struct MeshSrc {
   const T *gq_ = nullptr;  // gradient buffer (the viscous stage pass only)
   __device__ bool skip_copy(int it) const { return probe_ != 0 && it == 0; }
   __device__ uint32_t wait_limit() const { return probe_ ? PROBE_WAIT_LIMIT : WAIT_LIMIT; }
-  __device__ void begin(unsigned char *) {}
+  __device__ void begin(unsigned char *) { grid_wait(Qin_, Qout_, rhs_, gq_); }
   __device__ void prefetch() {}
   __device__ void publish(int) {}
   __device__ int64_t g(int it) const { return (int64_t)blockIdx.x + (int64_t)it * gridDim.x; }
@@ -259,7 +259,6 @@ k_stage_pipe2(Src src, PhysT<T> p, T rka) {
     if constexpr (!AFF) rag(ds, sg, nv * PP::SB, last, &barT[b], true);
   };
 
-  src.begin(smem_raw + PP::smem());
   if (tid == 0) {
     for (int b = 0; b < PP::NSB + PP::NTB; ++b) mbar_init(&barS[b], 1);
     fence_mbar_init();
@@ -267,6 +266,7 @@ k_stage_pipe2(Src src, PhysT<T> p, T rka) {
   if constexpr (PP::MV > Nq)
     for (size_t t = tid; t < (size_t)DIM * PP::FDIR; t += C::THREADS)
       if ((int)(t % RS) >= Nq) sF[t] = T(0);
+  src.begin(smem_raw + PP::smem());
   __syncthreads();
   if (tid == 0)
     for (int j = 0; j < PP::LOOK && src.valid(j); ++j) {
