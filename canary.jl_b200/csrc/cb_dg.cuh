@@ -136,27 +136,9 @@ __device__ __forceinline__ T pressure(const T *q, T gc, const PhysT<T> &p) {
   return p.eos * ((q[IE] - ke / (T(2) * rho)) - rho * p.grav * gc);
 }
 
-// Euler flux f[s][c] (state s in reference order, direction c).
-template <int DIM, typename T>
-__device__ __forceinline__ void euler_flux(const T *q, T P, T (*f)[DIM]) {
-  constexpr int IR = Lay<DIM>::IR, IE = Lay<DIM>::IE;
-  const T ri = T(1) / q[IR];
-#pragma unroll
-  for (int a = 0; a < DIM; ++a) {
-#pragma unroll
-    for (int c = 0; c < DIM; ++c) {
-      T v = ri * q[a] * q[c];
-      if (a == c) v = v + P;
-      f[a][c] = v;
-    }
-    f[IR][a] = q[a];
-    f[IE][a] = ri * q[a] * (q[IE] + P);
-  }
-}
-
-// Variants for the fused stage: 1/ρ is formed once per state and reused by the
-// pressure, the fluxes and the wave speed (one FP64 division per state
-// instead of two; rounding differs from the reference's `/(2ρ)` by <= 1 ulp).
+// Pressure with 1/ρ formed once per state and reused by the fluxes and the wave
+// speed (one FP64 division per state instead of two; rounding differs from the
+// reference's `/(2ρ)` by <= 1 ulp).
 template <int DIM, typename T>
 __device__ __forceinline__ T pressure_ri(const T *q, T ri, T gc, const PhysT<T> &p) {
   constexpr int IR = Lay<DIM>::IR, IE = Lay<DIM>::IE;
@@ -179,33 +161,8 @@ __device__ __forceinline__ void euler_flux_ri(const T *q, T ri, T P, T (*f)[DIM]
     f[IE][a] = ri * q[a] * (q[IE] + P);
   }
 }
-template <int DIM, typename T>
-__device__ __forceinline__ void rusanov_ri(const T *qM, T rMi, T PM, const T *qP, T rPi, T PP,
-                                           const T *nrm, const PhysT<T> &p, T *out) {
-  constexpr int NS = Lay<DIM>::NS;
-  T fM[NS][DIM], fP[NS][DIM];
-  euler_flux_ri<DIM, T>(qM, rMi, PM, fM);
-  euler_flux_ri<DIM, T>(qP, rPi, PP, fP);
-  T unM = nrm[0] * qM[0] + nrm[1] * qM[1];
-  T unP = nrm[0] * qP[0] + nrm[1] * qP[1];
-  if (DIM == 3) {
-    unM = unM + nrm[2] * qM[2];
-    unP = unP + nrm[2] * qP[2];
-  }
-  const T lM = rMi * fabs(unM) + sqrt(rMi * p.gamma * PM);
-  const T lP = rPi * fabs(unP) + sqrt(rPi * p.gamma * PP);
-  T lam = lM > lP ? lM : lP;
-  if (lM != lM || lP != lP) lam = lM + lP;
-#pragma unroll
-  for (int s = 0; s < NS; ++s) {
-    T a = nrm[0] * (fM[s][0] + fP[s][0]) + nrm[1] * (fM[s][1] + fP[s][1]);
-    if (DIM == 3) a = a + nrm[2] * (fM[s][2] + fP[s][2]);
-    out[s] = (a - lam * (qP[s] - qM[s])) * T(0.5);
-  }
-}
-
 // Normal Euler flux n·F of one state (5 values) given 1/ρ and P: the
-// fused stage uses it instead of forming both 3x5 flux tensors and dotting
+// kernels use it instead of forming both 3x5 flux tensors and dotting
 // them with n (same mathematics, about a third of the operations).
 template <int DIM, typename T>
 __device__ __forceinline__ void normal_flux(const T *q, T ri, T P, const T *nrm, T &un, T *fn) {
@@ -240,34 +197,6 @@ __device__ __forceinline__ void rusanov_n(const T *qM, T rMi, T PM, const T *qP,
   if (lM != lM || lP != lP) lam = lM + lP;
 #pragma unroll
   for (int s = 0; s < NS; ++s) out[s] = ((fM[s] + fP[s]) - lam * (qP[s] - qM[s])) * T(0.5);
-}
-
-// Rusanov numerical flux (euler3d_set3c.jl:394-446): out[s] = n·(F⁻+F⁺)/2 - λ(q⁺-q⁻)/2
-template <int DIM, typename T>
-__device__ __forceinline__ void rusanov(const T *qM, T PM, const T *qP, T PP,
-                                        const T *nrm, const PhysT<T> &p,
-                                        T *out) {
-  constexpr int NS = Lay<DIM>::NS, IR = Lay<DIM>::IR;
-  T fM[NS][DIM], fP[NS][DIM];
-  euler_flux<DIM, T>(qM, PM, fM);
-  euler_flux<DIM, T>(qP, PP, fP);
-  const T rMi = T(1) / qM[IR], rPi = T(1) / qP[IR];
-  T unM = nrm[0] * qM[0] + nrm[1] * qM[1];
-  T unP = nrm[0] * qP[0] + nrm[1] * qP[1];
-  if (DIM == 3) {
-    unM = unM + nrm[2] * qM[2];
-    unP = unP + nrm[2] * qP[2];
-  }
-  const T lM = rMi * fabs(unM) + sqrt(rMi * p.gamma * PM);
-  const T lP = rPi * fabs(unP) + sqrt(rPi * p.gamma * PP);
-  T lam = lM > lP ? lM : lP;
-  if (lM != lM || lP != lP) lam = lM + lP;  // propagate NaN like Julia max
-#pragma unroll
-  for (int s = 0; s < NS; ++s) {
-    T a = nrm[0] * (fM[s][0] + fP[s][0]) + nrm[1] * (fM[s][1] + fP[s][1]);
-    if (DIM == 3) a = a + nrm[2] * (fM[s][2] + fP[s][2]);
-    out[s] = (a - lam * (qP[s] - qM[s])) / T(2);
-  }
 }
 
 // --------------------------------------------------------------- indexing
@@ -395,31 +324,7 @@ __device__ __forceinline__ void load_metric(const T *__restrict__ vg, int n,
 // Pointwise inviscid phase: contravariant fluxes of one node into sF and the
 // buoyancy source into R (euler3d_set3c.jl:274-324).
 template <int DIM, int Nq, int EPB, typename T>
-__device__ __forceinline__ void pointwise_euler(const T *q, const T *__restrict__ vg,
-                                                int n, int el, T *sF,
-                                                const PhysT<T> &p, T *R) {
-  constexpr int NS = Lay<DIM>::NS, Np = ipow(Nq, DIM), SP = EPB * Np;
-  constexpr int IR = Lay<DIM>::IR;
-  T met[DIM][DIM], MJ;
-  load_metric<DIM, T>(vg, n, Np, met, MJ);
-  const T gc = p.grav != T(0) ? vg[n + Np * (DIM * DIM + 2 + DIM - 1)] : T(0);
-  const T P = pressure<DIM, T>(q, gc, p);
-  T f[NS][DIM];
-  euler_flux<DIM, T>(q, P, f);
-#pragma unroll
-  for (int r = 0; r < DIM; ++r)
-#pragma unroll
-    for (int s = 0; s < NS; ++s) {
-      T a = met[r][0] * f[s][0] + met[r][1] * f[s][1];
-      if (DIM == 3) a = a + met[r][2] * f[s][2];
-      sF[(r * NS + s) * SP + el * Np + n] = MJ * a;
-    }
-  R[DIM - 1] -= MJ * q[IR] * p.grav;
-}
-
-// The same from the contravariant flux (contravariant_flux).
-template <int DIM, int Nq, int EPB, typename T>
-__device__ __forceinline__ void pointwise_euler_n(const T *q, const T *__restrict__ vg, int n, int el, T *sF,
+__device__ __forceinline__ void pointwise_euler(const T *q, const T *__restrict__ vg, int n, int el, T *sF,
                                                   const PhysT<T> &p, T *R) {
   constexpr int NS = Lay<DIM>::NS, Np = ipow(Nq, DIM), SP = EPB * Np, IR = Lay<DIM>::IR;
   T met[DIM][DIM], MJ;

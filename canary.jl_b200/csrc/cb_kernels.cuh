@@ -73,6 +73,24 @@ k_volumerhs(T *__restrict__ rhs, const T *__restrict__ Q,
   }
 }
 
+// Nodes of a face entry's 1-based ids: vM in element e, and element eP and node
+// vP of idP, eP = -1 if idP is not a node of the mesh (32-bit division where the
+// node count allows it).  Whether idM is a node of element e.
+__device__ __forceinline__ bool face_ids(int64_t idM, int64_t idP, int64_t e, int64_t nelem, int Np, int &vM,
+                                         int64_t &eP, int &vP) {
+  const int64_t oM = idM - 1 - e * Np, oP = idP - 1, all = nelem * Np;
+  vM = (int)oM;
+  if (all <= 0xffffffffll) {
+    eP = (uint32_t)oP / (uint32_t)Np;
+    vP = (int)((uint32_t)oP % (uint32_t)Np);
+  } else {
+    eP = oP / Np;
+    vP = (int)(oP % Np);
+  }
+  if (oP < 0 || oP >= all) eP = -1;
+  return oM >= 0 && oM < Np;
+}
+
 // ======================================================================
 // Stateless face RHS with the reference's int64 vmaps (fluxrhs!).
 // Face fluxes of the block's elements go to shared memory first and are then
@@ -88,7 +106,7 @@ k_fluxrhs(T *__restrict__ rhs, const T *__restrict__ Q,
           const int64_t *__restrict__ elemtobndy, PhysT<T> p,
           unsigned *status) {
   using C = Cfg<DIM, Nq>;
-  constexpr int NS = Lay<DIM>::NS, NVG = Lay<DIM>::NVG, NSG = Lay<DIM>::NSG;
+  constexpr int NS = Lay<DIM>::NS, NVG = Lay<DIM>::NVG, NSG = Lay<DIM>::NSG, IR = Lay<DIM>::IR;
   constexpr int Np = C::Np, Nfp = C::Nfp, NF = C::NFACE, FS = C::EPB * Nfp;
   constexpr int GC = DIM * DIM + 2 + DIM - 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -108,28 +126,32 @@ k_fluxrhs(T *__restrict__ rhs, const T *__restrict__ Q,
     for (int c = 0; c < DIM; ++c) nrm[c] = sg[c];
     const T sMJ = sg[DIM];
     const int64_t idM = vmapM[fidx], idP = vmapP[fidx];
-    const int64_t vM = (idM - 1) % Np, eP = (idP - 1) / Np, vP = (idP - 1) % Np;
-    T qM[NS], qP[NS];
-#pragma unroll
-    for (int s = 0; s < NS; ++s) qM[s] = Q[vM + Np * (s + NS * e)];
-    const T gM = p.grav != T(0) ? vgeo[vM + Np * (GC + NVG * e)] : T(0);
-    const T PM = pressure<DIM, T>(qM, gM, p);
-    T PP;
     const int64_t bc = elemtobndy[f + NF * e];
-    T out[NS];
-    if ((idM - 1) / Np != e || idM < 1 || (bc == 0 && (idP < 1 || eP >= nelem))) {
+    int vM, vP;
+    int64_t eP;
+    const bool mapped = face_ids(idM, idP, e, nelem, Np, vM, eP, vP);
+    if (!mapped || (bc == 0 && eP < 0)) {
       atomicOr(status, ST_MESH);  // vmapP points outside the mesh: skip the face
 #pragma unroll
       for (int s = 0; s < NS; ++s) FF[(f * NS + s) * FS + el * Nfp + fn] = T(0);
       continue;
     }
+    T qM[NS], qP[NS], out[NS];
+#pragma unroll
+    for (int s = 0; s < NS; ++s) qM[s] = Q[vM + Np * (s + NS * e)];
+    const T gM = p.grav != T(0) ? vgeo[vM + Np * (GC + NVG * e)] : T(0);
+    const T riM = T(1) / qM[IR];
+    const T PM = pressure_ri<DIM, T>(qM, riM, gM, p);
+    T PP, riP;
     if (bc == 0) {
 #pragma unroll
       for (int s = 0; s < NS; ++s) qP[s] = Q[vP + Np * (s + NS * eP)];
       const T gP = p.grav != T(0) ? vgeo[vP + Np * (GC + NVG * eP)] : T(0);
-      PP = pressure<DIM, T>(qP, gP, p);
+      riP = T(1) / qP[IR];
+      PP = pressure_ri<DIM, T>(qP, riP, gP, p);
     } else if (bc == 1) {
       wall_state<DIM, T>(qM, nrm, qP);
+      riP = riM;
       PP = PM;
     } else {
       atomicOr(status, ST_BC);
@@ -137,7 +159,7 @@ k_fluxrhs(T *__restrict__ rhs, const T *__restrict__ Q,
       for (int s = 0; s < NS; ++s) FF[(f * NS + s) * FS + el * Nfp + fn] = T(0);
       continue;
     }
-    rusanov<DIM, T>(qM, PM, qP, PP, nrm, p, out);
+    rusanov_n<DIM, T>(qM, riM, PM, qP, riP, PP, nrm, p, out);
 #pragma unroll
     for (int s = 0; s < NS; ++s) FF[(f * NS + s) * FS + el * Nfp + fn] = sMJ * out[s];
   }
@@ -163,22 +185,51 @@ k_fluxrhs(T *__restrict__ rhs, const T *__restrict__ Q,
 }
 
 // ======================================================================
-// Stateless update (updatesolution!).  Elementwise.
+// Stateless update (updatesolution!).  BY_NODE: one thread per node takes all
+// its fields, the index is divided once and eleven loads are in flight per
+// thread instead of three (B200, 2.3 M nodes, N=5: FP64 75.6 -> 66.5 us, FP32
+// 49.4 -> 33.1).  FP64 elements of fewer than 64 nodes take one thread per value:
+// a field of theirs is too short a run for a warp (N=2 FP64: 78 us by value, 99
+// by node).
 // ======================================================================
-template <int DIM, typename T>
-__global__ void k_update(T *__restrict__ rhs, const T *__restrict__ rhs_gradQ,
-                         T *__restrict__ Q, const T *__restrict__ vgeo,
-                         int64_t nelem, int Np, T rka, T rkb, T dt, T visc) {
-  constexpr int NS = Lay<DIM>::NS, NVG = Lay<DIM>::NVG, MJI = DIM * DIM + 1;
-  const int64_t total = (int64_t)Np * NS * nelem;
-  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total;
-       q += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t n = q % Np, e = q / ((int64_t)Np * NS);
-    const int s = (int)((q / Np) % NS);
-    T r = rhs[q];
-    if (rhs_gradQ) r += visc * rhs_gradQ[n + Np * (s + (int64_t)NS * DIM * e)];
-    Q[q] += rkb * dt * r * vgeo[n + Np * (MJI + (int64_t)NVG * e)];
-    rhs[q] = r * rka;
+template <int DIM, int Nq, typename T>
+constexpr bool update_by_node = sizeof(T) == 4 || ipow(Nq, DIM) >= 64;
+template <int DIM, int Nq, typename T>
+__global__ void __launch_bounds__(256) k_update(T *__restrict__ rhs, const T *__restrict__ rhs_gradQ,
+                                                T *__restrict__ Q, const T *__restrict__ vgeo, int64_t nelem, T rka,
+                                                T rkb, T dt, T visc) {
+  constexpr int NS = Lay<DIM>::NS, NVG = Lay<DIM>::NVG, MJI = DIM * DIM + 1, Np = ipow(Nq, DIM);
+  const int64_t g = blockIdx.x * (int64_t)256 + threadIdx.x;
+  if constexpr (!update_by_node<DIM, Nq, T>) {
+    if (g >= nelem * (Np * NS)) return;
+    const int64_t e = g / (Np * NS);
+    const int m = (int)(g - e * (Np * NS)), n = m % Np;
+    T r = rhs[g];
+    if (rhs_gradQ) r += visc * rhs_gradQ[m + e * (Np * NS * DIM)];
+    Q[g] += rkb * dt * r * vgeo[n + Np * (MJI + (int64_t)NVG * e)];
+    rhs[g] = r * rka;
+    return;
+  }
+  if (g >= nelem * Np) return;
+  const int64_t e = g / Np;
+  const int n = (int)(g - e * Np);
+  T *r0 = rhs + n + e * (Np * NS), *q0 = Q + n + e * (Np * NS);
+  T r[NS], q[NS];
+#pragma unroll
+  for (int s = 0; s < NS; ++s) {
+    r[s] = r0[Np * s];
+    q[s] = q0[Np * s];
+  }
+  const T mji = vgeo[n + Np * (MJI + (int64_t)NVG * e)];
+  if (rhs_gradQ) {
+    const T *v = rhs_gradQ + n + e * ((int64_t)Np * NS * DIM);
+#pragma unroll
+    for (int s = 0; s < NS; ++s) r[s] += visc * v[Np * s];
+  }
+#pragma unroll
+  for (int s = 0; s < NS; ++s) {
+    q0[Np * s] = q[s] + rkb * dt * r[s] * mji;
+    r0[Np * s] = r[s] * rka;
   }
 }
 
@@ -226,7 +277,7 @@ k_stage(const T *Qin_, T *Qout_, T *rhs_,
         q[s] = d + qref.v[s];
         R[u][s] = rhs[n + Np * (s + NS * e)];
       }
-      pointwise_euler_n<DIM, Nq, C::EPB, T>(q, vgeo + (int64_t)Np * NVG * e, n, el, sF, p, R[u]);
+      pointwise_euler<DIM, Nq, C::EPB, T>(q, vgeo + (int64_t)Np * NVG * e, n, el, sF, p, R[u]);
     }
   }
   __syncthreads();
@@ -447,14 +498,17 @@ k_flux_grad(T *__restrict__ rhs, const T *__restrict__ Q,
     for (int c = 0; c < DIM; ++c) nrm[c] = sg[c];
     const T sMJ = sg[DIM];
     const int64_t idM = vmapM[fidx], idP = vmapP[fidx];
-    const int64_t vM = (idM - 1) % Np, eP = (idP - 1) / Np, vP = (idP - 1) % Np;
+    int vM, vP;
+    int64_t eP;
+    const bool mapped = face_ids(idM, idP, e, nelem, Np, vM, eP, vP);
+    if (!mapped) vM = 0;
     T qM[NS], pM[NS], pP[NS];
 #pragma unroll
     for (int s = 0; s < NS; ++s) qM[s] = Q[vM + Np * (s + NS * e)];
     const T gM = p.grav != T(0) ? vgeo[vM + Np * (GC + NVG * e)] : T(0);
     primitives<DIM, T>(qM, gM, p, pM);
     const int64_t bc = elemtobndy[f + NF * e];
-    if ((idM - 1) / Np != e || idM < 1 || (bc == 0 && (idP < 1 || eP >= nelem))) {
+    if (!mapped || (bc == 0 && eP < 0)) {
       atomicOr(status, ST_MESH);
       for (int s = 0; s < NS * DIM; ++s) FF[(f * NS * DIM + s) * FS + el * Nfp + fn] = T(0);
       continue;
@@ -509,17 +563,19 @@ k_flux_grad(T *__restrict__ rhs, const T *__restrict__ Q,
   }
 }
 
-// update_gradQ!: gradQ = rhs * MJI (elementwise)
-template <int DIM, typename T>
-__global__ void k_update_gradQ(T *__restrict__ gradQ, const T *__restrict__ rhs,
-                               const T *__restrict__ vgeo, int64_t nelem, int Np) {
-  constexpr int NS = Lay<DIM>::NS, NVG = Lay<DIM>::NVG, MJI = DIM * DIM + 1;
-  const int64_t total = (int64_t)Np * NS * DIM * nelem;
-  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total;
-       q += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t n = q % Np, e = q / ((int64_t)Np * NS * DIM);
-    gradQ[q] = rhs[q] * vgeo[n + Np * (MJI + (int64_t)NVG * e)];
-  }
+// update_gradQ!: gradQ = rhs * MJI, one thread per node.
+template <int DIM, int Nq, typename T>
+__global__ void __launch_bounds__(256) k_update_gradQ(T *__restrict__ gradQ, const T *__restrict__ rhs,
+                                                      const T *__restrict__ vgeo, int64_t nelem) {
+  constexpr int NS = Lay<DIM>::NS, NVG = Lay<DIM>::NVG, MJI = DIM * DIM + 1, Np = ipow(Nq, DIM);
+  const int64_t g = blockIdx.x * (int64_t)256 + threadIdx.x;
+  if (g >= nelem * Np) return;
+  const int64_t e = g / Np;
+  const int n = (int)(g - e * Np);
+  const int64_t o = n + e * ((int64_t)Np * NS * DIM);
+  const T mji = vgeo[n + Np * (MJI + (int64_t)NVG * e)];
+#pragma unroll
+  for (int s = 0; s < NS * DIM; ++s) gradQ[o + Np * s] = rhs[o + Np * s] * mji;
 }
 
 // Viscous flux of one node (nse3d.jl:717-742 / nse2d.jl:598-614).
@@ -633,7 +689,10 @@ k_flux_div(T *__restrict__ rhs, const T *__restrict__ gradQ,
     for (int c = 0; c < DIM; ++c) nrm[c] = sg[c];
     const T sMJ = sg[DIM];
     const int64_t idM = vmapM[fidx], idP = vmapP[fidx];
-    const int64_t vM = (idM - 1) % Np, eP = (idP - 1) / Np, vP = (idP - 1) % Np;
+    int vM, vP;
+    int64_t eP;
+    const bool mapped = face_ids(idM, idP, e, nelem, Np, vM, eP, vP);
+    if (!mapped) vM = 0;
     T gm[NS][DIM], gp[NS][DIM], vM_[DIM], vP_[DIM];
 #pragma unroll
     for (int s = 0; s < NS; ++s)
@@ -643,7 +702,7 @@ k_flux_div(T *__restrict__ rhs, const T *__restrict__ gradQ,
 #pragma unroll
     for (int c = 0; c < DIM; ++c) vM_[c] = Q[vM + Np * (c + NS * e)] / rhoM;
     const int64_t bc = elemtobndy[f + NF * e];
-    if ((idM - 1) / Np != e || idM < 1 || (bc == 0 && (idP < 1 || eP >= nelem))) {
+    if (!mapped || (bc == 0 && eP < 0)) {
       atomicOr(status, ST_MESH);
       for (int s = 0; s < NS; ++s) FF[(f * NS + s) * FS + el * Nfp + fn] = T(0);
       continue;
@@ -790,6 +849,10 @@ struct Launch {
 
   static cudaError_t volumerhs(T *rhs, const T *Q, const T *vgeo, const T *D, int64_t nelem,
                                const PhysT<T> &p, cudaStream_t st) {
+    // 3-D N >= 3 (FP64: 4): the march (B200, 2.3 M nodes, us: FP64 N=4 98.9 ->
+    // 90.0, N=8 190.8 -> 166.2, N=10 188.6 -> 149.9, FP32 N=7 72.4 -> 57.9; below,
+    // the grouped kernel is the faster one: FP64 N=3 72.5, march 74.1)
+    if constexpr (DIM == 3 && Nq >= (sizeof(T) == 4 ? 4 : 5)) return march_volume<T>(Nq, rhs, Q, vgeo, D, nelem, p, st);
     size_t sm = smem_volume();
     cudaError_t err = prep(k_volumerhs<DIM, Nq, T>, sm);
     if (err != cudaSuccess) return err;

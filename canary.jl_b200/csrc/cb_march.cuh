@@ -82,6 +82,8 @@ struct March {
   // N=7 viscous stage step 3.06 ms at 168, 3.57 ms at 128)
   static constexpr int REGS_STAGE = sizeof(T) == 4 ? (Nq <= 5 ? 96 : Nq <= 8 ? 128 : 168) : (Nq <= 5 ? 168 : 255);
   static constexpr int REGS_NS = sizeof(T) == 4 ? (Nq <= 5 ? 128 : 168) : 255;
+  static constexpr int REGS_VOLUME = sizeof(T) == 4 ? (Nq <= 8 ? 96 : 128) : (Nq <= 5 ? 128 : Nq <= 8 ? 168 : 255);
+  static constexpr size_t smem_volume() { return OFF_FF; }
   static constexpr int REGS_GRAD = sizeof(T) == 4 ? (Nq <= 5 ? 96 : 128) : (Nq <= 8 ? 168 : 255);
 };
 
@@ -407,6 +409,95 @@ __global__ void __launch_bounds__(March<Nq, T>::THREADS,
   if (bad) atomicOr(a.status, ST_NONFINITE);
 }
 
+// The volume integral alone (volumerhs!): the march without faces and update,
+// rhs += volume terms.  The grouped kernel reads every flux value Nq times per
+// direction from shared memory and is bound by that pipe (3-D N=5 FP64, 2.3 M
+// nodes: 96 us, 84 % of its wavefronts).
+template <int Nq, typename T>
+__global__ void __launch_bounds__(March<Nq, T>::THREADS, March<Nq, T>::blocks_for(March<Nq, T>::REGS_VOLUME))
+    k_march_volume(T *__restrict__ rhs_, const T *__restrict__ Q_, const T *__restrict__ vgeo, const T *__restrict__ D,
+                   int64_t nelem, PhysT<T> p) {
+  using C = March<Nq, T>;
+  constexpr int Np = C::Np, N2 = C::N2, NS = 5, NVG = 14, IR = 3, RS = C::RS, ROW = C::ROW, MJF = 9, GC = 13, EPB = C::EPB;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  T *DT = reinterpret_cast<T *>(smem_raw + C::OFF_DT), *DZ = reinterpret_cast<T *>(smem_raw + C::OFF_DZ);
+  T *PL = reinterpret_cast<T *>(smem_raw + C::OFF_P);
+  const int tid = threadIdx.x, el = tid / N2, ij = tid % N2, i = ij % Nq, j = ij / Nq;
+  const int64_t e0 = (int64_t)blockIdx.x * EPB, e = e0 + el;
+  const bool act = el < EPB && e < nelem;
+  const int64_t ec = act ? e : e0;
+  const T *__restrict__ Q = Q_ + ec * (Np * NS) + ij;
+  const T *__restrict__ vg = vgeo + ec * (Np * NVG) + ij;
+  T *__restrict__ rhs = rhs_ + ec * (Np * NS) + ij;
+  T q[NS], m[9], MJ, hz = T(0);
+  auto load_plane = [&](int k) {
+#pragma unroll
+    for (int s = 0; s < NS; ++s) q[s] = ld_here(Q + N2 * k + Np * s);
+#pragma unroll
+    for (int c = 0; c < 9; ++c) m[c] = ld_here(vg + N2 * k + Np * c);
+    MJ = ld_here(vg + N2 * k + Np * MJF);
+    if (p.grav != T(0)) hz = vg[N2 * k + Np * GC];
+  };
+  load_plane(0);
+  march_load_D<Nq, RS, C::THREADS, T>(DT, DZ, D);
+  T acc[Nq][NS];
+#pragma unroll
+  for (int k = 0; k < Nq; ++k)
+#pragma unroll
+    for (int s = 0; s < NS; ++s) acc[k][s] = ld_here(rhs + N2 * k + Np * s);
+  __syncthreads();  // D
+  T dx[C::DREG ? Nq : 1], dy[C::DREG ? Nq : 1];
+  if constexpr (C::DREG) {
+    march_row<Nq, T>(DT + i * RS, dx);
+    march_row<Nq, T>(DT + j * RS, dy);
+  }
+  const int elr = (act ? el : 0) * Nq;
+#pragma unroll
+  for (int k = 0; k < Nq; ++k) {
+    T *F = PL + (k & 1) * (2 * NS * ROW), *G = F + NS * ROW;
+    if (act) {
+      const T ri = T(1) / q[IR];
+      const T P = pressure_ri<3, T>(q, ri, hz, p);
+      T f[3][NS];
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+        const T row[3] = {m[r], m[r + 3], m[r + 6]};
+        contravariant_flux<3, T>(q, ri, P, MJ, row, f[r]);
+      }
+      acc[k][2] -= MJ * q[IR] * p.grav;
+#pragma unroll
+      for (int s = 0; s < NS; ++s) {
+        F[s * ROW + (elr + j) * RS + i] = f[0][s];
+        G[s * ROW + (elr + i) * RS + j] = f[1][s];
+      }
+      if (k + 1 < Nq) load_plane(k + 1);
+      T dz[Nq];
+      march_row<Nq, T>(DZ + k * RS, dz);
+#pragma unroll
+      for (int x = 0; x < Nq; ++x)
+#pragma unroll
+        for (int s = 0; s < NS; ++s) acc[x][s] += dz[x] * f[2][s];
+    }
+    __syncthreads();
+    if (act) {
+      T d[Nq];
+      if constexpr (!C::DREG) march_row<Nq, T>(DT + i * RS, d);
+#pragma unroll
+      for (int s = 0; s < NS; ++s)
+        acc[k][s] = march_dot<Nq, T>(F + s * ROW + (elr + j) * RS, C::DREG ? dx : d, acc[k][s]);
+      if constexpr (!C::DREG) march_row<Nq, T>(DT + j * RS, d);
+#pragma unroll
+      for (int s = 0; s < NS; ++s)
+        acc[k][s] = march_dot<Nq, T>(G + s * ROW + (elr + i) * RS, C::DREG ? dy : d, acc[k][s]);
+    }
+  }
+  if (!act) return;
+#pragma unroll
+  for (int k = 0; k < Nq; ++k)
+#pragma unroll
+    for (int s = 0; s < NS; ++s) rhs[N2 * k + Np * s] = acc[k][s];
+}
+
 // Node x of the thread's line in direction R in a slab with rows of QR.
 template <int Nq, int QR, int R>
 __device__ __forceinline__ int line_slab(int a, int b, int x) {
@@ -612,6 +703,18 @@ struct MarchLaunch {
     return visc ? launch(k_march_stage<Nq, T, true>, M::smem_stage(), a, p, st)
                 : launch(k_march_stage<Nq, T, false>, M::smem_stage(), a, p, st);
   }
+  static cudaError_t volume(T *rhs, const T *Q, const T *vgeo, const T *D, int64_t nelem, const PhysT<T> &p,
+                            cudaStream_t st) {
+    const int64_t g = (nelem + M::EPB - 1) / M::EPB;
+    if (g <= 0) return cudaSuccess;
+    if (M::smem_volume() > 48 * 1024) {
+      const cudaError_t e = cudaFuncSetAttribute(k_march_volume<Nq, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 (int)M::smem_volume());
+      if (e != cudaSuccess) return e;
+    }
+    k_march_volume<Nq, T><<<(unsigned)g, M::THREADS, M::smem_volume(), st>>>(rhs, Q, vgeo, D, nelem, p);
+    return cudaGetLastError();
+  }
   static cudaError_t grad(const MarchArgs<T> &a, const PhysT<T> &p, cudaStream_t st) {
     return launch(k_line_grad<Nq, T>, M::smem_grad(), a, p, st);
   }
@@ -630,6 +733,17 @@ struct MarchLaunch {
         &MarchLaunch<8, T_>::stage, &MarchLaunch<9, T_>::stage, &MarchLaunch<10, T_>::stage,                        \
         &MarchLaunch<11, T_>::stage};                                                                               \
     return Nq < 2 || Nq > 11 ? cudaErrorInvalidValue : f[Nq - 2](visc, a, p, st);                                   \
+  }                                                                                                                 \
+  template <>                                                                                                       \
+  cudaError_t march_volume<T_>(int Nq, T_ *rhs, const T_ *Q, const T_ *vgeo, const T_ *D, int64_t nelem,            \
+                               const PhysT<T_> &p, cudaStream_t st) {                                               \
+    static cudaError_t (*const f[])(T_ *, const T_ *, const T_ *, const T_ *, int64_t, const PhysT<T_> &,           \
+                                    cudaStream_t) = {                                                               \
+        &MarchLaunch<2, T_>::volume, &MarchLaunch<3, T_>::volume, &MarchLaunch<4, T_>::volume,                      \
+        &MarchLaunch<5, T_>::volume, &MarchLaunch<6, T_>::volume, &MarchLaunch<7, T_>::volume,                      \
+        &MarchLaunch<8, T_>::volume, &MarchLaunch<9, T_>::volume, &MarchLaunch<10, T_>::volume,                     \
+        &MarchLaunch<11, T_>::volume};                                                                              \
+    return Nq < 2 || Nq > 11 ? cudaErrorInvalidValue : f[Nq - 2](rhs, Q, vgeo, D, nelem, p, st);                    \
   }                                                                                                                 \
   template <>                                                                                                       \
   cudaError_t march_grad<T_>(int Nq, const MarchArgs<T_> &a, const PhysT<T_> &p, cudaStream_t st) {                 \

@@ -24,6 +24,10 @@ struct MarchArgs {
 // gradient pass.
 template <typename T>
 cudaError_t march_stage(int Nq, bool visc, const MarchArgs<T> &a, const PhysT<T> &p, cudaStream_t st);
+// rhs += volume integral (volumerhs!).
+template <typename T>
+cudaError_t march_volume(int Nq, T *rhs, const T *Q, const T *vgeo, const T *D, int64_t nelem, const PhysT<T> &p,
+                         cudaStream_t st);
 template <typename T>
 cudaError_t march_grad(int Nq, const MarchArgs<T> &a, const PhysT<T> &p, cudaStream_t st);
 

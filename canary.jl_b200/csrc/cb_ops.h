@@ -47,7 +47,7 @@ struct Ops {
                             cudaStream_t);
   cudaError_t (*flux_div)(T *, const T *, const T *, const T *, int64_t, const int64_t *, const int64_t *,
                           const int64_t *, const PhysT<T> &, unsigned *, cudaStream_t);
-  // order-independent element-wise kernels
+  // element-wise kernels (the int is the node count of an element)
   cudaError_t (*update)(T *, const T *, T *, const T *, int64_t, int, T, T, T, T, cudaStream_t);
   cudaError_t (*update_gradQ)(T *, const T *, const T *, int64_t, int, cudaStream_t);
   cudaError_t (*cons_sums)(const T *, const T *, int64_t, int, const Offs<double, 5> &, double *, int,
