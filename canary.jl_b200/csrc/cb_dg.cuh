@@ -35,10 +35,10 @@ __device__ __forceinline__ void grid_wait(P *&...ptr) {
 }
 template <typename... K, typename... A>
 inline cudaError_t launch_stage_kernel(void (*kernel)(K...), unsigned grid, int threads, size_t smem, cudaStream_t st,
-                                       const A &...args) {
+                                       int programmatic, const A &...args) {
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
+  at.val.programmaticStreamSerializationAllowed = programmatic;
   cudaLaunchConfig_t c{};
   c.gridDim = dim3(grid);
   c.blockDim = dim3(threads);
@@ -324,11 +324,9 @@ __device__ __forceinline__ void load_metric(const T *__restrict__ vg, int n,
 // Pointwise inviscid phase: contravariant fluxes of one node into sF and the
 // buoyancy source into R (euler3d_set3c.jl:274-324).
 template <int DIM, int Nq, int EPB, typename T>
-__device__ __forceinline__ void pointwise_euler(const T *q, const T *__restrict__ vg, int n, int el, T *sF,
-                                                  const PhysT<T> &p, T *R) {
+__device__ __forceinline__ void pointwise_euler(const T *q, const T (*met)[DIM], T MJ, const T *__restrict__ vg, int n,
+                                                int el, T *sF, const PhysT<T> &p, T *R) {
   constexpr int NS = Lay<DIM>::NS, Np = ipow(Nq, DIM), SP = EPB * Np, IR = Lay<DIM>::IR;
-  T met[DIM][DIM], MJ;
-  load_metric<DIM, T>(vg, n, Np, met, MJ);
   const T gc = p.grav != T(0) ? vg[n + Np * (DIM * DIM + 2 + DIM - 1)] : T(0);
   const T ri = T(1) / q[IR];
   const T P = pressure_ri<DIM, T>(q, ri, gc, p);

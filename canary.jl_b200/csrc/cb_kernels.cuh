@@ -56,7 +56,10 @@ k_volumerhs(T *__restrict__ rhs, const T *__restrict__ Q,
         q[s] = Q[n + Np * (s + NS * e)];
         R[u][s] = rhs[n + Np * (s + NS * e)];
       }
-      pointwise_euler<DIM, Nq, C::EPB, T>(q, vgeo + (int64_t)Np * NVG * e, n, el, sF, p, R[u]);
+      T met[DIM][DIM], MJ;
+      const T *vg = vgeo + (int64_t)Np * NVG * e;
+      load_metric<DIM, T>(vg, n, Np, met, MJ);
+      pointwise_euler<DIM, Nq, C::EPB, T>(q, met, MJ, vg, n, el, sF, p, R[u]);
     }
   }
   __syncthreads();
@@ -238,8 +241,12 @@ __global__ void __launch_bounds__(256) k_update(T *__restrict__ rhs, const T *__
 //   Qin   state at the start of the stage (read, also for neighbour traces)
 //   Qout  state after the stage (distinct buffer)
 //   rhs   residual carry: read, then overwritten with rka_next * residual
+// EARLY: for launches of a block or two per SM, whose time is one block's
+// latency: metric, normals and neighbour codes are loaded before the wait for
+// the preceding stage and the neighbours' traces with the state, at the price of
+// registers that a full SM could not spare (see Launch::EARLY_BLOCKS).
 // ======================================================================
-template <int DIM, int Nq, typename T>
+template <int DIM, int Nq, typename T, bool EARLY = false>
 __global__ void __launch_bounds__(Cfg<DIM, Nq>::THREADS)
 k_stage(const T *Qin_, T *Qout_, T *rhs_,
         const T *__restrict__ vgeo, const T *__restrict__ sgeo,
@@ -256,11 +263,50 @@ k_stage(const T *Qin_, T *Qout_, T *rhs_,
   T *sQ = Ds + ((Nq * Nq + 1) & ~1);  // [NS][SP]
   T *sF = sQ + NS * SP;               // [DIM][NS][SP], reused as FF
   load_D(Ds, D, Nq * Nq);
+  const int64_t e0 = ebeg + (int64_t)blockIdx.x * C::EPB;
+  // EARLY: what no stage writes, while the preceding one finishes
+  T met[EARLY ? C::NPT : 1][DIM][DIM], MJ[EARLY ? C::NPT : 1], mjis[EARLY ? C::NPT : 1];
+  int32_t nbs[EARLY ? C::FPT : 1];
+  T nrms[EARLY ? C::FPT : 1][DIM + 1], qNb[EARLY ? C::FPT : 1][NS];
+  if constexpr (EARLY) {
+#pragma unroll
+    for (int u = 0; u < C::NPT; ++u) {
+      const int slot = threadIdx.x + u * C::THREADS;
+      const int el = slot / Np, n = slot % Np;
+      if (slot < C::SLOTS && e0 + el < nelem) {
+        const T *vg = vgeo + (int64_t)Np * NVG * (e0 + el);
+        load_metric<DIM, T>(vg, n, Np, met[u], MJ[u]);
+        mjis[u] = vg[n + Np * MJI];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < C::FPT; ++u) {
+      const int fs = threadIdx.x + u * C::THREADS;
+      const int el = fs / (NF * Nfp), f = (fs / Nfp) % NF, fn = fs % Nfp;
+      nbs[u] = NBR_WALL;
+      if (fs < C::FSLOTS && e0 + el < nelem) {
+        nbs[u] = nbr[f + NF * (e0 + el)];
+        const T *sg = sgeo + (int64_t)NSG * (fn + (int64_t)Nfp * (f + NF * (e0 + el)));
+#pragma unroll
+        for (int c = 0; c <= DIM; ++c) nrms[u][c] = sg[c];
+      }
+    }
+  }
   grid_wait(Qin_, Qout_, rhs_);
   const T *__restrict__ Qin = Qin_;
   T *__restrict__ Qout = Qout_;
   T *__restrict__ rhs = rhs_;
-  const int64_t e0 = ebeg + (int64_t)blockIdx.x * C::EPB;
+  if constexpr (EARLY) {  // the neighbours' traces, in flight with the state
+#pragma unroll
+    for (int u = 0; u < C::FPT; ++u) {
+      const int fn = (threadIdx.x + u * C::THREADS) % Nfp;
+      if (nbs[u] >= 0) {
+        const T *q2 = Qin + face_node<DIM, Nq>(nbs[u] & 7, fn) + (int64_t)(nbs[u] >> 3) * (Np * NS);
+#pragma unroll
+        for (int s = 0; s < NS; ++s) qNb[u][s] = q2[Np * s];
+      }
+    }
+  }
   T R[C::NPT][NS];
   // ---- pointwise fluxes
 #pragma unroll
@@ -277,7 +323,14 @@ k_stage(const T *Qin_, T *Qout_, T *rhs_,
         q[s] = d + qref.v[s];
         R[u][s] = rhs[n + Np * (s + NS * e)];
       }
-      pointwise_euler<DIM, Nq, C::EPB, T>(q, vgeo + (int64_t)Np * NVG * e, n, el, sF, p, R[u]);
+      const T *vg = vgeo + (int64_t)Np * NVG * e;
+      if constexpr (EARLY) {
+        pointwise_euler<DIM, Nq, C::EPB, T>(q, met[u], MJ[u], vg, n, el, sF, p, R[u]);
+      } else {
+        T m[DIM][DIM], mj;
+        load_metric<DIM, T>(vg, n, Np, m, mj);
+        pointwise_euler<DIM, Nq, C::EPB, T>(q, m, mj, vg, n, el, sF, p, R[u]);
+      }
     }
   }
   __syncthreads();
@@ -302,21 +355,21 @@ k_stage(const T *Qin_, T *Qout_, T *rhs_,
     const T *sg = sgeo + (int64_t)NSG * (fn + (int64_t)Nfp * (f + NF * e));
     T nrm[DIM];
 #pragma unroll
-    for (int c = 0; c < DIM; ++c) nrm[c] = sg[c];
-    const T sMJ = sg[DIM];
+    for (int c = 0; c < DIM; ++c) nrm[c] = EARLY ? nrms[EARLY ? u : 0][c] : sg[c];
+    const T sMJ = EARLY ? nrms[EARLY ? u : 0][DIM] : sg[DIM];
     T qM[NS], qP[NS];
 #pragma unroll
     for (int s = 0; s < NS; ++s) qM[s] = sQ[s * SP + el * Np + vM] + qref.v[s];
     const T gM = p.grav != T(0) ? vgeo[vM + Np * (GC + NVG * e)] : T(0);
     const T riM = T(1) / qM[IR];
     const T PM = pressure_ri<DIM, T>(qM, riM, gM, p);
-    const int32_t nb = nbr[f + NF * e];
+    const int32_t nb = EARLY ? nbs[EARLY ? u : 0] : nbr[f + NF * e];
     T PP, riP;
     if (nb >= 0) {
       const int64_t e2 = nb >> 3;
       const int vP = face_node<DIM, Nq>(nb & 7, fn);
 #pragma unroll
-      for (int s = 0; s < NS; ++s) qP[s] = Qin[vP + Np * (s + NS * e2)] + qref.v[s];
+      for (int s = 0; s < NS; ++s) qP[s] = (EARLY ? qNb[EARLY ? u : 0][s] : Qin[vP + Np * (s + NS * e2)]) + qref.v[s];
       const T gP = p.grav != T(0) ? vgeo[vP + Np * (GC + NVG * e2)] : T(0);
       riP = T(1) / qP[IR];
       PP = pressure_ri<DIM, T>(qP, riP, gP, p);
@@ -340,7 +393,7 @@ k_stage(const T *Qin_, T *Qout_, T *rhs_,
     const int64_t e = e0 + el;
     if (slot < C::SLOTS && e < nelem) {
       gather_face_terms<DIM, Nq, C::EPB, T>(FF, el, n, R[u]);
-      const T mji = vgeo[n + Np * (MJI + (int64_t)NVG * e)];
+      const T mji = EARLY ? mjis[EARLY ? u : 0] : vgeo[n + Np * (MJI + (int64_t)NVG * e)];
 #pragma unroll
       for (int s = 0; s < NS; ++s) {
         const T qn = sQ[s * SP + slot] + rkbdt * R[u][s] * mji;
@@ -902,6 +955,13 @@ struct Launch {
       : DIM == 3 && (Nq <= 3 || (sizeof(T) == 4 && Nq <= 10)) ? 3
       : 1;
   static constexpr bool LEAN_DEFAULT = DEFAULT_KERNEL == 4;
+  // Small launches of the shapes that default to the grouped stage, and of 2-D,
+  // run its EARLY form: up to EARLY_BLOCKS blocks per SM.
+  static constexpr bool EARLY_OK = C::NPT == 1 && !MARCH && (DIM == 2 || DEFAULT_KERNEL == 3);
+  // (us a stage, stages in a row on one solver: FP32 3-D N=3 8^3 4.9 -> 3.0, 12^3
+  // 6.4 -> 5.6, N=4 8^3 5.9 -> 4.4, N=6 6^3 6.8 -> 5.3, 2-D N=4 48^2 5.7 -> 3.2;
+  // FP64 2-D N=4 10^2 4.9 -> 2.9, but N=7 32^2 4.5 at one block, 5.6 at two)
+  static constexpr int EARLY_BLOCKS = sizeof(T) == 4 ? 4 : 1;
   // Resident blocks per SM of a kernel at `smem` bytes, from the occupancy
   // calculator, cached per device in `cache`.
   template <typename K>
@@ -959,6 +1019,15 @@ struct Launch {
     if (kernel == 4 && !aligned2) kernel = 1;  // bulk copies need 16-byte aligned slabs
     const int64_t groups = (nelem - ebeg + C::EPB - 1) / C::EPB;
     if (groups == 0) return cudaSuccess;
+    if constexpr (EARLY_OK) {
+      if ((grouped_default || (DIM == 2 && kernel == 0 && !probe && !ebeg)) && groups <= EARLY_BLOCKS * num_sms()) {
+        const size_t sm = smem_stage();
+        const cudaError_t err = prep(k_stage<DIM, Nq, T, true>, sm);
+        if (err != cudaSuccess) return err;
+        return launch_stage_kernel(k_stage<DIM, Nq, T, true>, (unsigned)groups, C::THREADS, sm, st, 1, Qin, Qout, rhs,
+                                   vgeo, sgeo, nbr, D, nelem, p, qref, rka, rkbdt, status, ebeg);
+      }
+    }
     if constexpr (MMA_OK) {
       if ((kernel == 2 || (kernel == 0 && MMA_DEFAULT)) && aligned2) {
         using S = MeshSrc<T, NS, C::EPB>;  // MeshSrc<T, 5, 1> here
@@ -970,7 +1039,7 @@ struct Launch {
         int64_t g = (int64_t)num_sms() * bps;
         if (g > groups) g = groups;
         const S src{Qin, Qout, rhs, vgeo, sgeo, nbr, D, nelem, qref, rkbdt, status, probe, ebeg};
-        return launch_stage_kernel(k_stage_mma<S, PM::MINB>, (unsigned)g, PM::THREADS, PM::smem(), st, src, p, rka);
+        return launch_stage_kernel(k_stage_mma<S, PM::MINB>, (unsigned)g, PM::THREADS, PM::smem(), st, 1, src, p, rka);
       }
     }
     if constexpr (LEAN_OK) {
@@ -984,7 +1053,7 @@ struct Launch {
         int64_t g = (int64_t)num_sms() * bps;
         if (g > groups) g = groups;
         const S src{Qin, Qout, rhs, vgeo, sgeo, nbr, D, nelem, qref, rkbdt, status, probe, ebeg};
-        return launch_stage_kernel(k_stage_lean<DIM, Nq, T, S>, (unsigned)g, C::THREADS, PL::smem(), st, src, p, rka);
+        return launch_stage_kernel(k_stage_lean<DIM, Nq, T, S>, (unsigned)g, C::THREADS, PL::smem(), st, 1, src, p, rka);
       }
     }
     if (Pipe2<DIM, Nq, T>::OK && aligned2 && kernel != 3) {
@@ -998,7 +1067,7 @@ struct Launch {
       int64_t g = (int64_t)num_sms() * bps;
       if (g > groups) g = groups;
       const S src{Qin, Qout, rhs, vgeo, sgeo, nbr, D, nelem, qref, rkbdt, status, probe, ebeg};
-      return launch_stage_kernel(k_stage_pipe2<DIM, Nq, T, S>, (unsigned)g, C::THREADS, sm, st, src, p, rka);
+      return launch_stage_kernel(k_stage_pipe2<DIM, Nq, T, S>, (unsigned)g, C::THREADS, sm, st, 1, src, p, rka);
     } else if (probe || (ebeg && !grouped_default)) {
       return cudaErrorNotSupported;
     } else if (pipe_ok && aligned && kernel != 3) {
@@ -1015,7 +1084,9 @@ struct Launch {
       size_t sm = smem_stage();
       cudaError_t err = prep(k_stage<DIM, Nq, T>, sm);
       if (err != cudaSuccess) return err;
-      return launch_stage_kernel(k_stage<DIM, Nq, T>, (unsigned)groups, C::THREADS, sm, st, Qin, Qout, rhs, vgeo, sgeo,
+      // (plain up to a wave: the next stage's blocks would crowd onto the SMs that
+      // have room, FP32 N=4 10^3: 9.5 us a stage against 7.6)
+      return launch_stage_kernel(k_stage<DIM, Nq, T>, (unsigned)groups, C::THREADS, sm, st, groups > 8 * num_sms(), Qin, Qout, rhs, vgeo, sgeo,
                                  nbr, D, nelem, p, qref, rka, rkbdt, status, ebeg);
     }
   }

@@ -697,7 +697,7 @@ struct MarchLaunch {
       const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return e;
     }
-    return launch_stage_kernel(kernel, (unsigned)g, M::THREADS, smem, st, a, p);
+    return launch_stage_kernel(kernel, (unsigned)g, M::THREADS, smem, st, 1, a, p);
   }
   static cudaError_t stage(bool visc, const MarchArgs<T> &a, const PhysT<T> &p, cudaStream_t st) {
     return visc ? launch(k_march_stage<Nq, T, true>, M::smem_stage(), a, p, st)
