@@ -23,7 +23,9 @@ namespace cb {
 // grid_wait (all threads, before anything that a stage writes is read or
 // written) returns once the preceding grid is complete and its writes visible;
 // only then is the dependent grid let go, so that no grid starts while the one
-// two before it still reads the buffer which it will read.  The pointers depend
+// two before it still reads the buffer which it will read.  Only a launch that
+// directly follows a pass of the same solve is programmatic (chained): what else
+// may precede it in the stream can write the geometry.  The pointers depend
 // on the instruction: loads from them (read-only data to the compiler) cannot be
 // moved above it.  Both instructions do nothing in a plain launch.
 template <typename... P>

@@ -989,12 +989,13 @@ struct Launch {
   // test hook of the pipelined, lean and tensor-core stages (see MeshSrc);
   // shapes without one return cudaErrorNotSupported for it.
   // ebeg: the launch covers elements ebeg .. nelem - 1 (neighbour indices
-  // stay absolute); only the pipelined, lean and tensor-core stages take
-  // ebeg > 0, the others return cudaErrorNotSupported for it.
+  // stay absolute); only the pipelined, lean and tensor-core stages and the
+  // default column march and grouped stage take ebeg > 0, the others return cudaErrorNotSupported for it.  chained: the
+  // stream's preceding launch is a stage of the same solve (see grid_wait).
   static cudaError_t stage(const T *Qin, T *Qout, T *rhs, const T *vgeo, const T *sgeo,
                            const int32_t *nbr, const T *D, int64_t nelem, const PhysT<T> &p,
                            const Offs<T, NS> &qref, T rka, T rkbdt, unsigned *status,
-                           cudaStream_t st, int probe = 0, int kernel = 0, int64_t ebeg = 0) {
+                           cudaStream_t st, int probe = 0, int kernel = 0, int64_t ebeg = 0, int chained = 0) {
     constexpr bool pipe_ok = Pipe<DIM, Nq, T>::OK;
     const bool aligned = ((reinterpret_cast<uintptr_t>(Qin) | reinterpret_cast<uintptr_t>(vgeo)) & 15) == 0;
     const bool aligned2 = aligned && ((reinterpret_cast<uintptr_t>(rhs) | reinterpret_cast<uintptr_t>(sgeo)) & 15) == 0;
@@ -1003,7 +1004,7 @@ struct Launch {
       if (!probe && (kernel == 0 || (kernel == 3 && !ebeg))) {
         MarchArgs<T> a{Qin, Qout, rhs, vgeo, sgeo, nbr, D, nullptr, ebeg, nelem, {}, rka, rkbdt, status};
         for (int s = 0; s < NS; ++s) a.qref.v[s] = qref.v[s];
-        return march_stage<T>(Nq, false, a, p, st);
+        return march_stage<T>(Nq, false, a, p, st, chained);
       }
     }
     // the shape's default; the grouped stage takes no test hook: that call
@@ -1024,8 +1025,8 @@ struct Launch {
         const size_t sm = smem_stage();
         const cudaError_t err = prep(k_stage<DIM, Nq, T, true>, sm);
         if (err != cudaSuccess) return err;
-        return launch_stage_kernel(k_stage<DIM, Nq, T, true>, (unsigned)groups, C::THREADS, sm, st, 1, Qin, Qout, rhs,
-                                   vgeo, sgeo, nbr, D, nelem, p, qref, rka, rkbdt, status, ebeg);
+        return launch_stage_kernel(k_stage<DIM, Nq, T, true>, (unsigned)groups, C::THREADS, sm, st, chained, Qin, Qout,
+                                   rhs, vgeo, sgeo, nbr, D, nelem, p, qref, rka, rkbdt, status, ebeg);
       }
     }
     if constexpr (MMA_OK) {
@@ -1039,7 +1040,7 @@ struct Launch {
         int64_t g = (int64_t)num_sms() * bps;
         if (g > groups) g = groups;
         const S src{Qin, Qout, rhs, vgeo, sgeo, nbr, D, nelem, qref, rkbdt, status, probe, ebeg};
-        return launch_stage_kernel(k_stage_mma<S, PM::MINB>, (unsigned)g, PM::THREADS, PM::smem(), st, 1, src, p, rka);
+        return launch_stage_kernel(k_stage_mma<S, PM::MINB>, (unsigned)g, PM::THREADS, PM::smem(), st, chained, src, p, rka);
       }
     }
     if constexpr (LEAN_OK) {
@@ -1053,7 +1054,7 @@ struct Launch {
         int64_t g = (int64_t)num_sms() * bps;
         if (g > groups) g = groups;
         const S src{Qin, Qout, rhs, vgeo, sgeo, nbr, D, nelem, qref, rkbdt, status, probe, ebeg};
-        return launch_stage_kernel(k_stage_lean<DIM, Nq, T, S>, (unsigned)g, C::THREADS, PL::smem(), st, 1, src, p, rka);
+        return launch_stage_kernel(k_stage_lean<DIM, Nq, T, S>, (unsigned)g, C::THREADS, PL::smem(), st, chained, src, p, rka);
       }
     }
     if (Pipe2<DIM, Nq, T>::OK && aligned2 && kernel != 3) {
@@ -1067,7 +1068,7 @@ struct Launch {
       int64_t g = (int64_t)num_sms() * bps;
       if (g > groups) g = groups;
       const S src{Qin, Qout, rhs, vgeo, sgeo, nbr, D, nelem, qref, rkbdt, status, probe, ebeg};
-      return launch_stage_kernel(k_stage_pipe2<DIM, Nq, T, S>, (unsigned)g, C::THREADS, sm, st, 1, src, p, rka);
+      return launch_stage_kernel(k_stage_pipe2<DIM, Nq, T, S>, (unsigned)g, C::THREADS, sm, st, chained, src, p, rka);
     } else if (probe || (ebeg && !grouped_default)) {
       return cudaErrorNotSupported;
     } else if (pipe_ok && aligned && kernel != 3) {
@@ -1086,8 +1087,8 @@ struct Launch {
       if (err != cudaSuccess) return err;
       // (plain up to a wave: the next stage's blocks would crowd onto the SMs that
       // have room, FP32 N=4 10^3: 9.5 us a stage against 7.6)
-      return launch_stage_kernel(k_stage<DIM, Nq, T>, (unsigned)groups, C::THREADS, sm, st, groups > 8 * num_sms(), Qin, Qout, rhs, vgeo, sgeo,
-                                 nbr, D, nelem, p, qref, rka, rkbdt, status, ebeg);
+      return launch_stage_kernel(k_stage<DIM, Nq, T>, (unsigned)groups, C::THREADS, sm, st, chained && groups > 8 * num_sms(),
+                                 Qin, Qout, rhs, vgeo, sgeo, nbr, D, nelem, p, qref, rka, rkbdt, status, ebeg);
     }
   }
   // Whether stage() takes an element range (ebeg > 0) for arrays aligned

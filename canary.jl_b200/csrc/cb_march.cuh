@@ -690,18 +690,19 @@ template <int Nq, typename T>
 struct MarchLaunch {
   using M = March<Nq, T>;
   template <typename K>
-  static cudaError_t launch(K kernel, size_t smem, const MarchArgs<T> &a, const PhysT<T> &p, cudaStream_t st) {
+  static cudaError_t launch(K kernel, size_t smem, const MarchArgs<T> &a, const PhysT<T> &p, cudaStream_t st,
+                            int chained) {
     const int64_t g = (a.eend - a.ebeg + M::EPB - 1) / M::EPB;
     if (g <= 0) return cudaSuccess;
     if (smem > 48 * 1024) {
       const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return e;
     }
-    return launch_stage_kernel(kernel, (unsigned)g, M::THREADS, smem, st, 1, a, p);
+    return launch_stage_kernel(kernel, (unsigned)g, M::THREADS, smem, st, chained, a, p);
   }
-  static cudaError_t stage(bool visc, const MarchArgs<T> &a, const PhysT<T> &p, cudaStream_t st) {
-    return visc ? launch(k_march_stage<Nq, T, true>, M::smem_stage(), a, p, st)
-                : launch(k_march_stage<Nq, T, false>, M::smem_stage(), a, p, st);
+  static cudaError_t stage(bool visc, const MarchArgs<T> &a, const PhysT<T> &p, cudaStream_t st, int chained) {
+    return visc ? launch(k_march_stage<Nq, T, true>, M::smem_stage(), a, p, st, chained)
+                : launch(k_march_stage<Nq, T, false>, M::smem_stage(), a, p, st, chained);
   }
   static cudaError_t volume(T *rhs, const T *Q, const T *vgeo, const T *D, int64_t nelem, const PhysT<T> &p,
                             cudaStream_t st) {
@@ -715,8 +716,8 @@ struct MarchLaunch {
     k_march_volume<Nq, T><<<(unsigned)g, M::THREADS, M::smem_volume(), st>>>(rhs, Q, vgeo, D, nelem, p);
     return cudaGetLastError();
   }
-  static cudaError_t grad(const MarchArgs<T> &a, const PhysT<T> &p, cudaStream_t st) {
-    return launch(k_line_grad<Nq, T>, M::smem_grad(), a, p, st);
+  static cudaError_t grad(const MarchArgs<T> &a, const PhysT<T> &p, cudaStream_t st, int chained) {
+    return launch(k_line_grad<Nq, T>, M::smem_grad(), a, p, st, chained);
   }
 };
 
@@ -726,13 +727,14 @@ struct MarchLaunch {
 #define CB_MARCH_DEFINE(T_)                                                                                         \
   namespace cb {                                                                                                    \
   template <>                                                                                                       \
-  cudaError_t march_stage<T_>(int Nq, bool visc, const MarchArgs<T_> &a, const PhysT<T_> &p, cudaStream_t st) {     \
-    static cudaError_t (*const f[])(bool, const MarchArgs<T_> &, const PhysT<T_> &, cudaStream_t) = {               \
+  cudaError_t march_stage<T_>(int Nq, bool visc, const MarchArgs<T_> &a, const PhysT<T_> &p, cudaStream_t st,       \
+                              int chained) {                                                                        \
+    static cudaError_t (*const f[])(bool, const MarchArgs<T_> &, const PhysT<T_> &, cudaStream_t, int) = {          \
         &MarchLaunch<2, T_>::stage, &MarchLaunch<3, T_>::stage, &MarchLaunch<4, T_>::stage,                         \
         &MarchLaunch<5, T_>::stage, &MarchLaunch<6, T_>::stage, &MarchLaunch<7, T_>::stage,                         \
         &MarchLaunch<8, T_>::stage, &MarchLaunch<9, T_>::stage, &MarchLaunch<10, T_>::stage,                        \
         &MarchLaunch<11, T_>::stage};                                                                               \
-    return Nq < 2 || Nq > 11 ? cudaErrorInvalidValue : f[Nq - 2](visc, a, p, st);                                   \
+    return Nq < 2 || Nq > 11 ? cudaErrorInvalidValue : f[Nq - 2](visc, a, p, st, chained);                          \
   }                                                                                                                 \
   template <>                                                                                                       \
   cudaError_t march_volume<T_>(int Nq, T_ *rhs, const T_ *Q, const T_ *vgeo, const T_ *D, int64_t nelem,            \
@@ -746,11 +748,11 @@ struct MarchLaunch {
     return Nq < 2 || Nq > 11 ? cudaErrorInvalidValue : f[Nq - 2](rhs, Q, vgeo, D, nelem, p, st);                    \
   }                                                                                                                 \
   template <>                                                                                                       \
-  cudaError_t march_grad<T_>(int Nq, const MarchArgs<T_> &a, const PhysT<T_> &p, cudaStream_t st) {                 \
-    static cudaError_t (*const f[])(const MarchArgs<T_> &, const PhysT<T_> &, cudaStream_t) = {                     \
+  cudaError_t march_grad<T_>(int Nq, const MarchArgs<T_> &a, const PhysT<T_> &p, cudaStream_t st, int chained) {    \
+    static cudaError_t (*const f[])(const MarchArgs<T_> &, const PhysT<T_> &, cudaStream_t, int) = {                \
         &MarchLaunch<2, T_>::grad, &MarchLaunch<3, T_>::grad, &MarchLaunch<4, T_>::grad, &MarchLaunch<5, T_>::grad, \
         &MarchLaunch<6, T_>::grad, &MarchLaunch<7, T_>::grad, &MarchLaunch<8, T_>::grad, &MarchLaunch<9, T_>::grad, \
         &MarchLaunch<10, T_>::grad, &MarchLaunch<11, T_>::grad};                                                    \
-    return Nq < 2 || Nq > 11 ? cudaErrorInvalidValue : f[Nq - 2](a, p, st);                                         \
+    return Nq < 2 || Nq > 11 ? cudaErrorInvalidValue : f[Nq - 2](a, p, st, chained);                                \
   }                                                                                                                 \
   }

@@ -21,14 +21,14 @@ struct MarchArgs {
 };
 
 // Fused stage of order Nq - 1 (visc: the second viscous pass) and the
-// gradient pass.
+// gradient pass (chained: see launch_stage_kernel).
 template <typename T>
-cudaError_t march_stage(int Nq, bool visc, const MarchArgs<T> &a, const PhysT<T> &p, cudaStream_t st);
+cudaError_t march_stage(int Nq, bool visc, const MarchArgs<T> &a, const PhysT<T> &p, cudaStream_t st, int chained);
 // rhs += volume integral (volumerhs!).
 template <typename T>
 cudaError_t march_volume(int Nq, T *rhs, const T *Q, const T *vgeo, const T *D, int64_t nelem, const PhysT<T> &p,
                          cudaStream_t st);
 template <typename T>
-cudaError_t march_grad(int Nq, const MarchArgs<T> &a, const PhysT<T> &p, cudaStream_t st);
+cudaError_t march_grad(int Nq, const MarchArgs<T> &a, const PhysT<T> &p, cudaStream_t st, int chained);
 
 }  // namespace cb

@@ -25,9 +25,10 @@ struct Ops {
   // cudaErrorNotSupported where no pipelined stage runs), the kernel choice
   // (0 the shape's default, 1 the CUDA-core stages, 2 the tensor-core stage;
   // cudaErrorNotSupported where the choice is not built) and the first
-  // element of the launch (elements first .. nelem - 1)
+  // element of the launch (elements first .. nelem - 1), and whether the
+  // stream's preceding launch is a stage of the same solve (see grid_wait)
   cudaError_t (*stage_k)(const T *, T *, T *, const T *, const T *, const int32_t *, const T *, int64_t,
-                         const PhysT<T> &, const Offs<T, 5> &, T, T, unsigned *, cudaStream_t, int, int, int64_t);
+                         const PhysT<T> &, const Offs<T, 5> &, T, T, unsigned *, cudaStream_t, int, int, int64_t, int);
   // whether stage_k takes a first element > 0 (an element range) for arrays
   // aligned like these: (Qin, rhs, vgeo, sgeo)
   bool (*ranged)(const void *, const void *, const void *, const void *);
@@ -53,8 +54,9 @@ struct Ops {
   cudaError_t (*cons_sums)(const T *, const T *, int64_t, int, const Offs<double, 5> &, double *, int,
                            cudaStream_t);
   // fused viscous passes over one mesh: pass 0 (gradient) or 1 (stage +
-  // update); the last argument is the solver's kernel choice
-  cudaError_t (*ns_pass)(int, const BDesc<T> &, T *, int64_t, const PhysT<T> &, T, T, cudaStream_t, int);
+  // update); the last arguments are the solver's kernel choice and whether the
+  // stream's preceding launch is a pass of the same solve
+  cudaError_t (*ns_pass)(int, const BDesc<T> &, T *, int64_t, const PhysT<T> &, T, T, cudaStream_t, int, int);
   // whether the viscous form of this order has stage calls, ghosts and state
   // offsets (every 2-D order, 3-D N <= 7)
   bool ns_stage_form;

@@ -84,8 +84,9 @@ unsigned *visc_status(const cb_solver *s) { return ns_stage_form(s) ? s->status 
 // the state ping-pongs between Q and Qalt (two steps per graph)
 bool pingpong(const cb_solver *s) { return s->phys.visc <= 0 || fused_visc(s); }
 
+// One step; chained: the stream's preceding launch is the step before it.
 template <typename T>
-cudaError_t enqueue_step(cb_solver *s, double dt, bool from_user) {
+cudaError_t enqueue_step(cb_solver *s, double dt, bool from_user, bool chained) {
   const Ops<T> *o = ops<T>(s);
   const PhysT<T> p(Phys{s->phys.gamma, s->phys.R_gas, s->phys.c_p, s->phys.c_v, s->phys.gravity,
                         s->phys.Pr, s->phys.lambda, s->phys.visc});
@@ -105,8 +106,11 @@ cudaError_t enqueue_step(cb_solver *s, double dt, bool from_user) {
     for (int st = 0; st < 5 && e == cudaSuccess; ++st) {
       I.Q[0] = a;
       I.Q[1] = b;
-      if ((e = o->ns_pass(0, I, (T *)s->gradQ, s->nelem, p, T(0), T(0), s->stream, s->kernel)) != cudaSuccess) break;
-      e = o->ns_pass(1, I, (T *)s->gradQ, s->nelem, p, T(RKA[(st + 1) % 5]), T(RKB[st] * dt), s->stream, s->kernel);
+      if ((e = o->ns_pass(0, I, (T *)s->gradQ, s->nelem, p, T(0), T(0), s->stream, s->kernel,
+                          chained || st)) != cudaSuccess)
+        break;
+      e = o->ns_pass(1, I, (T *)s->gradQ, s->nelem, p, T(RKA[(st + 1) % 5]), T(RKB[st] * dt), s->stream, s->kernel,
+                     1);
       T *t = a;
       a = b;
       b = t;
@@ -132,7 +136,7 @@ cudaError_t enqueue_step(cb_solver *s, double dt, bool from_user) {
   for (int k = 0; k < 5; ++k) q5.v[k] = T(s->qref[k]);
   for (int st = 0; st < 5 && e == cudaSuccess; ++st) {
     e = o->stage_k(a, b, (T *)s->rhs, vg, sg, s->nbr, D, s->nelem, p, q5, T(RKA[(st + 1) % 5]),
-                   T(RKB[st] * dt), s->status, s->stream, 0, s->kernel, 0);
+                   T(RKB[st] * dt), s->status, s->stream, 0, s->kernel, 0, chained || st);
     T *t = a;
     a = b;
     b = t;
@@ -140,8 +144,9 @@ cudaError_t enqueue_step(cb_solver *s, double dt, bool from_user) {
   return e;
 }
 
-cudaError_t enqueue(cb_solver *s, double dt, bool from_user) {
-  return s->prec == 64 ? enqueue_step<double>(s, dt, from_user) : enqueue_step<float>(s, dt, from_user);
+cudaError_t enqueue(cb_solver *s, double dt, bool from_user, bool chained) {
+  return s->prec == 64 ? enqueue_step<double>(s, dt, from_user, chained)
+                       : enqueue_step<float>(s, dt, from_user, chained);
 }
 
 void drop_graph(cb_solver *s) {
@@ -158,8 +163,8 @@ int capture(cb_solver *s, double dt, int reps, cudaGraphExec_t *exec) {
   if (e != cudaSuccess) return solver_fail(CB_ERR_CUDA, "begin capture: %s", cudaGetErrorString(e));
   cudaError_t e1 = cudaSuccess;
   for (int r = 0; r < reps && e1 == cudaSuccess; ++r) {
-    e1 = enqueue(s, dt, true);
-    if (pingpong(s) && e1 == cudaSuccess) e1 = enqueue(s, dt, false);  // two steps
+    e1 = enqueue(s, dt, true, r > 0);
+    if (pingpong(s) && e1 == cudaSuccess) e1 = enqueue(s, dt, false, true);  // two steps
   }
   cudaGraph_t graph = nullptr;
   e = cudaStreamEndCapture(s->stream, &graph);
@@ -210,15 +215,15 @@ cudaError_t enqueue_pass(cb_solver *s, int st, double dt, int pass) {
     I.status = visc_status(s);
     I.dt = dt;
     for (int k = 0; k < 5; ++k) I.qref[k] = T(s->qref[k]);
-    return pass == 0 ? o->ns_pass(0, I, (T *)s->gradQ, s->nelem, p, T(0), T(0), s->stream, s->kernel)
+    return pass == 0 ? o->ns_pass(0, I, (T *)s->gradQ, s->nelem, p, T(0), T(0), s->stream, s->kernel, 0)
                      : o->ns_pass(1, I, (T *)s->gradQ, s->nelem, p, T(RKA[(st + 1) % 5]), T(RKB[st] * dt), s->stream,
-                                  s->kernel);
+                                  s->kernel, 0);
   }
   if (pass == 0) return cudaSuccess;
   Offs<T, 5> q5;
   for (int k = 0; k < 5; ++k) q5.v[k] = T(s->qref[k]);
   return o->stage_k(a, b, (T *)s->rhs, (const T *)s->vgeo, (const T *)s->sgeo, s->nbr, (const T *)s->D, s->nelem,
-                    p, q5, T(RKA[(st + 1) % 5]), T(RKB[st] * dt), s->status, s->stream, 0, s->kernel, 0);
+                    p, q5, T(RKA[(st + 1) % 5]), T(RKB[st] * dt), s->status, s->stream, 0, s->kernel, 0, 0);
 }
 
 // The column-march passes (3-D) keep the gradient as records of 12 values per
@@ -337,14 +342,15 @@ int cb_solver_stage_split(cb_solver *s, int stage, double dt, int half, void **n
       for (int k = 0; k < 5; ++k) q5.v[k] = s->qref[k];
       e = ops<double>(s)->stage_k((const double *)a, (double *)b, (double *)s->rhs, (const double *)s->vgeo,
                                   (const double *)s->sgeo, s->nbr, (const double *)s->D, hi, PhysT<double>(ph), q5,
-                                  RKA[(stage + 1) % 5], RKB[stage] * dt, s->status, s->stream, 0, s->kernel, lo);
+                                  RKA[(stage + 1) % 5], RKB[stage] * dt, s->status, s->stream, 0, s->kernel, lo,
+                                  0);
     } else {
       Offs<float, 5> q5;
       for (int k = 0; k < 5; ++k) q5.v[k] = (float)s->qref[k];
       e = ops<float>(s)->stage_k((const float *)a, (float *)b, (float *)s->rhs, (const float *)s->vgeo,
                                  (const float *)s->sgeo, s->nbr, (const float *)s->D, hi, PhysT<float>(ph), q5,
                                  (float)RKA[(stage + 1) % 5], (float)(RKB[stage] * dt), s->status, s->stream, 0,
-                                 s->kernel, lo);
+                                 s->kernel, lo, 0);
     }
   }
   if (e != cudaSuccess) return solver_fail(CB_ERR_CUDA, "cb_solver_stage_split: %s", cudaGetErrorString(e));
@@ -578,7 +584,9 @@ int cb_lsrk_run(cb_solver *s, int64_t nsteps, double dt) {
     // do not) costs a good part of a step.  Once a solver has run long enough to
     // pay for its capture (about 0.3 ms), LONG_REPS graphs are launched as one.
     // 2-D N=4 10x10 FP64, 20 steps: 137 -> 131 us
-    const bool small = per_graph == 2 && state_bytes(s) <= (size_t)LONG_STATE;
+    cudaStreamCaptureStatus outer = cudaStreamCaptureStatusActive;  // (of the caller's own graph)
+    const bool small = per_graph == 2 && state_bytes(s) <= (size_t)LONG_STATE && (s->exec_long ||
+                       (cudaStreamIsCapturing(s->stream, &outer) == cudaSuccess && outer == cudaStreamCaptureStatusNone));
     for (int64_t r = 0; r < reps;) {
       if (small && !s->exec_long && s->reps_run + (reps - r) >= LONG_AFTER && reps - r >= LONG_REPS) {
         const int rc = capture(s, dt, LONG_REPS, &s->exec_long);
@@ -592,7 +600,7 @@ int cb_lsrk_run(cb_solver *s, int64_t nsteps, double dt) {
     }
   }
   if (rem) {
-    if ((e = enqueue(s, dt, true)) != cudaSuccess)
+    if ((e = enqueue(s, dt, true, false)) != cudaSuccess)
       return solver_fail(CB_ERR_CUDA, "step launch: %s", cudaGetErrorString(e));
     const int Nq = s->N + 1;
     const int64_t Np = s->dim == 2 ? (int64_t)Nq * Nq : (int64_t)Nq * Nq * Nq;
@@ -700,13 +708,13 @@ int cb_solver_test_timeout(cb_solver *s) {
     for (int k = 0; k < 5; ++k) q5.v[k] = s->qref[k];
     e = ops<double>(s)->stage_k((const double *)a, (double *)b, (double *)s->rhs, (const double *)s->vgeo,
                                 (const double *)s->sgeo, s->nbr, (const double *)s->D, s->nelem, p64, q5, RKA[1],
-                                RKB[0], s->status, s->stream, 1, s->kernel, 0);
+                                RKB[0], s->status, s->stream, 1, s->kernel, 0, 0);
   } else {
     Offs<float, 5> q5;
     for (int k = 0; k < 5; ++k) q5.v[k] = (float)s->qref[k];
     e = ops<float>(s)->stage_k((const float *)a, (float *)b, (float *)s->rhs, (const float *)s->vgeo,
                                (const float *)s->sgeo, s->nbr, (const float *)s->D, s->nelem, p32, q5,
-                               (float)RKA[1], (float)RKB[0], s->status, s->stream, 1, s->kernel, 0);
+                               (float)RKA[1], (float)RKB[0], s->status, s->stream, 1, s->kernel, 0, 0);
   }
   if (e == cudaErrorNotSupported)  // returned by the launcher, not by CUDA
     return solver_fail(CB_ERR_UNSUPPORTED, "cb_solver_test_timeout: this shape does not run the pipelined stage");
