@@ -933,10 +933,11 @@ struct Launch {
   // Whether the unpipelined choice (3) and the default are the column march
   // (cb_march.cuh) instead of the grouped stage: where the all-at-once plan
   // leaves one block per SM (B200, one mesh of 5.8-6.5 M nodes, ms per step:
-  // N=10 FP64 4.28 -> 3.35, FP32 1.92 -> 1.61; N=9 FP64 2.96 -> 2.72).  Below,
+  // N=10 FP64 4.28 -> 3.35, FP32 1.92 -> 1.61; N=9 FP64 2.96 -> 2.72; N=8 FP64
+  // 16^3 1.58 -> 1.43, under gravity 1.64 -> 1.45).  Below,
   // the other stages are the faster ones (N=9 FP32 grouped 1.36, march 1.51;
   // N=4 FP32 1.21, 1.24; N=7 FP64 tensor-core 1.75, march 2.34).
-  static constexpr bool MARCH = DIM == 3 && (Nq >= 11 || (Nq == 10 && sizeof(T) == 8));
+  static constexpr bool MARCH = DIM == 3 && (Nq >= 11 || (Nq >= 9 && sizeof(T) == 8));
   // Default stage kernel per shape, from B200 timings of one mesh (ms per
   // step, warped 3-D cubes of 7-17 M nodes; pipelined CUDA-core / grouped /
   // lean): FP64 N=3 3.66 / 3.34 / 2.76, N=4 4.95 / 4.20 / 3.78, N=5 2.37 /

@@ -37,16 +37,18 @@ namespace cb {
 
 // Elements per block: the lines of EPB elements fill the block's warps (threads
 // in use: 32·4, 14·9, 8·16, 5·25, 5·36, 3·49, 2·64, 81, 100, 121).  FP64 takes
-// fewer elements at N=5 and 6 (3·36, 2·49), where the registers of the larger
-// block leave one block per SM.
+// fewer elements at N=5, 6 and 7 (2·36, 49, 64): of its 230 to 255 registers a
+// thread, few large blocks fit an SM (B200, ms per viscous step: N=5 20^3 three
+// elements 2.58, two 2.18, four 2.30; N=6 17^3 two 2.15, one 2.06; N=7 16^3 two
+// 2.54, one 2.40).
 __host__ __device__ constexpr int march_epb(int nq, int w) {
   return nq == 2   ? 32
          : nq == 3 ? 14
          : nq == 4 ? 8
          : nq == 5 ? 5
-         : nq == 6 ? (w == 4 ? 5 : 3)
-         : nq == 7 ? (w == 4 ? 3 : 2)
-         : nq == 8 ? 2
+         : nq == 6 ? (w == 4 ? 5 : 2)
+         : nq == 7 ? (w == 4 ? 3 : 1)
+         : nq == 8 ? (w == 4 ? 2 : 1)
                    : 1;
 }
 
@@ -78,13 +80,15 @@ struct March {
   static constexpr bool DREG = sizeof(T) * Nq <= 48;
   // resident blocks the registers are sized for
   static constexpr int blocks_for(int regs) { return 65536 / (THREADS * regs) < 1 ? 1 : 65536 / (THREADS * regs); }
-  // (fewer registers and more blocks spill; more registers lose a block: FP32
+  // (fewer registers and more blocks spill; more registers lose a block: FP64
+  // N=8 16^3 inviscid step 1.68 ms at 255, 1.43 ms at 168, the lean stage 1.58;
+  // viscous passes at 168 instead of 255: N=4 2.06 -> 2.69, N=9 2.31 -> 2.96; FP32
   // N=7 viscous stage step 3.06 ms at 168, 3.57 ms at 128)
-  static constexpr int REGS_STAGE = sizeof(T) == 4 ? (Nq <= 5 ? 96 : Nq <= 8 ? 128 : 168) : (Nq <= 5 ? 168 : 255);
-  static constexpr int REGS_NS = sizeof(T) == 4 ? (Nq <= 5 ? 128 : 168) : 255;
+  static constexpr int REGS_STAGE = sizeof(T) == 4 ? (Nq <= 5 ? 96 : Nq <= 8 ? 128 : 168) : (Nq <= 5 || Nq == 9 ? 168 : 255);
+  static constexpr int REGS_NS = sizeof(T) == 4 ? (Nq <= 5 ? 128 : 168) : Nq == 6 ? 224 : 255;
   static constexpr int REGS_VOLUME = sizeof(T) == 4 ? (Nq <= 8 ? 96 : 128) : (Nq <= 5 ? 128 : Nq <= 8 ? 168 : 255);
   static constexpr size_t smem_volume() { return OFF_FF; }
-  static constexpr int REGS_GRAD = sizeof(T) == 4 ? (Nq <= 5 ? 96 : 128) : (Nq <= 8 ? 168 : 255);
+  static constexpr int REGS_GRAD = sizeof(T) == 4 ? (Nq <= 5 ? 96 : 128) : (Nq <= 9 ? 168 : 255);
 };
 
 // Loads that stay where the march issues them (volatile), ahead of the barrier
@@ -480,15 +484,16 @@ __global__ void __launch_bounds__(March<Nq, T>::THREADS, March<Nq, T>::blocks_fo
     }
     __syncthreads();
     if (act) {
-      T d[Nq];
+      // the ξ and η terms are summed by themselves: each cancels to a small value
+      // (the rows of D have the sum 0), the ζ sum is half done
+      T d[Nq], t[NS];
       if constexpr (!C::DREG) march_row<Nq, T>(DT + i * RS, d);
 #pragma unroll
-      for (int s = 0; s < NS; ++s)
-        acc[k][s] = march_dot<Nq, T>(F + s * ROW + (elr + j) * RS, C::DREG ? dx : d, acc[k][s]);
+      for (int s = 0; s < NS; ++s) t[s] = march_dot<Nq, T>(F + s * ROW + (elr + j) * RS, C::DREG ? dx : d, T(0));
       if constexpr (!C::DREG) march_row<Nq, T>(DT + j * RS, d);
 #pragma unroll
       for (int s = 0; s < NS; ++s)
-        acc[k][s] = march_dot<Nq, T>(G + s * ROW + (elr + i) * RS, C::DREG ? dy : d, acc[k][s]);
+        acc[k][s] += march_dot<Nq, T>(G + s * ROW + (elr + i) * RS, C::DREG ? dy : d, t[s]);
     }
   }
   if (!act) return;

@@ -190,7 +190,7 @@ int cb_solver_status_async(cb_solver *s, unsigned *out_host);
  * DMMA tiles, for FP32 solvers on the FP32 fluxes converted to FP64, the sum
  * rounded once; built for 3-D N=7, CB_ERR_UNSUPPORTED elsewhere), 3 = the
  * unpipelined grouped stages (the inviscid k_stage, the column march at 3-D
- * N=10 and FP64 N=9; for the fused viscous form the grouped passes), 4 = the lean
+ * N=10 and FP64 N=8, 9; for the fused viscous form the grouped passes), 4 = the lean
  * pipelined stage of the inviscid form (only the state staged in shared
  * memory, the geometry and carry read from L2; bit-identical to 1).  The
  * default is the fastest on B200 for the shape (viscous 3-D: the grid-line
