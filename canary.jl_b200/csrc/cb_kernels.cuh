@@ -952,10 +952,16 @@ struct Launch {
   static constexpr int DEFAULT_KERNEL =
       MARCH         ? 3
       : MMA_DEFAULT ? 2
-      : DIM == 3 && sizeof(T) == 8 && LEAN_OK && (Nq == 4 || Nq == 5 || Nq == 9) ? 4
+      : DIM == 3 && sizeof(T) == 8 && LEAN_OK && (Nq == 4 || Nq == 5) ? 4
       : DIM == 3 && (Nq <= 3 || (sizeof(T) == 4 && Nq <= 10)) ? 3
       : 1;
-  static constexpr bool LEAN_DEFAULT = DEFAULT_KERNEL == 4;
+  // The same under gravity, whose heights are a dependent load in every phase:
+  // where more warps are in flight than in the default (B200, ms per step: FP64
+  // N=6 19^3 pipelined 1.12, lean 1.08, without gravity 1.00 and 1.04; N=4 28^3
+  // lean 1.39, grouped 1.33, without gravity 1.30 and 1.32).
+  static constexpr int GRAVITY_KERNEL = DIM == 3 && sizeof(T) == 8 && Nq == 7   ? 4
+                                        : DIM == 3 && sizeof(T) == 8 && Nq == 5 ? 3
+                                                                                : DEFAULT_KERNEL;
   // Small launches of the shapes that default to the grouped stage, and of 2-D,
   // run its EARLY form: up to EARLY_BLOCKS blocks per SM.
   static constexpr bool EARLY_OK = C::NPT == 1 && !MARCH && (DIM == 2 || DEFAULT_KERNEL == 3);
@@ -1011,11 +1017,14 @@ struct Launch {
     // the shape's default; the grouped stage takes no test hook: that call
     // takes the pipelined stage, or the lean one where the pipelined plan does
     // not fit shared memory (3-D N=10 FP32)
-    const bool grouped_default = kernel == 0 && DEFAULT_KERNEL == 3 && !probe;
+    const int dflt = p.grav != T(0) && !probe ? GRAVITY_KERNEL : DEFAULT_KERNEL;
+    const bool grouped_default = kernel == 0 && dflt == 3 && !probe;
     if (kernel == 0 && (probe || ebeg) && !grouped_default && (DEFAULT_KERNEL == 1 || DEFAULT_KERNEL == 3))
       kernel = (Pipe2<DIM, Nq, T>::OK || !LEAN_OK) ? 1 : 4;
     else if (grouped_default)
       kernel = 3;
+    else if (kernel == 0 && dflt == 4)
+      kernel = 4;
     if (kernel == 2 && !(MMA_OK && aligned2)) return cudaErrorNotSupported;
     if (kernel == 4 && !LEAN_OK) return cudaErrorNotSupported;
     if (kernel == 4 && !aligned2) kernel = 1;  // bulk copies need 16-byte aligned slabs
@@ -1045,7 +1054,7 @@ struct Launch {
       }
     }
     if constexpr (LEAN_OK) {
-      if (kernel == 4 || (kernel == 0 && LEAN_DEFAULT && aligned2)) {
+      if (kernel == 4) {
         using S = MeshSrc<T, NS, C::EPB>;
         using PL = Lean<DIM, Nq, T>;
         static int per_sm[MAX_DEVICES] = {0};

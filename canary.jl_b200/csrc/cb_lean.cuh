@@ -44,7 +44,7 @@ struct Lean {
   static constexpr bool fits(int blocks) { return blocks * (smem() + RING_MAX + 1024) <= 228 * 1024; }
   // blocks of up to 256 threads: two (FP64) or three (FP32) per SM where
   // shared memory holds them
-  static constexpr int MINB = C::THREADS > 256 ? 1 : sizeof(T) == 8 ? (fits(2) ? 2 : 1) : (fits(3) ? 3 : fits(2) ? 2 : 1);
+  static constexpr int MINB = C::THREADS > (sizeof(T) == 8 ? 352 : 256) ? 1 : sizeof(T) == 8 ? (fits(2) ? 2 : 1) : (fits(3) ? 3 : fits(2) ? 2 : 1);
   static constexpr bool OK = smem() + RING_MAX <= SMEM_LIMIT;
 };
 
@@ -147,6 +147,8 @@ k_stage_lean(Src src, PhysT<T> p, T rka) {
     T *__restrict__ rhs = src.rhs(it) + e0 * Np * NS;
     // this group's metric (+ MJ, MJI), carry and face geometry into L2
     for (int el = 0; el < nv; ++el) prefetch_lines_l2(vg + el * Np * NVG, sizeof(T) * Np * (MJIF + 1));
+    if (Nq >= 7 && p.grav != T(0))  // and the heights
+      for (int el = 0; el < nv; ++el) prefetch_lines_l2(vg + Np * (GC + el * NVG), sizeof(T) * Np);
     prefetch_lines_l2(rhs, sizeof(T) * nv * Np * NS);
     prefetch_lines_l2(sg, sizeof(T) * nv * SE);
     T qr[NS];

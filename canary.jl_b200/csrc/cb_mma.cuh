@@ -161,6 +161,7 @@ __global__ void __launch_bounds__(PipeM::THREADS, MINB)
   auto prefetch_group = [&](int it) {  // thread 0 only: metric, carry, face geometry into L2
     const int64_t e = src.e0(it);
     prefetch_l2(src.vgeo(it) + e * Np * NVG, (uint32_t)PM::GB);
+    if (sizeof(T) == 8 && p.grav != T(0)) prefetch_l2(src.vgeo(it) + e * Np * NVG + Np * GC, (uint32_t)(sizeof(T) * Np));  // heights
     prefetch_l2(src.rhs(it) + e * Np * NS, (uint32_t)PM::QB);
     prefetch_l2(src.sgeo(it) + e * (int64_t)(NSG * Nfp * NF), (uint32_t)PM::SB);
   };

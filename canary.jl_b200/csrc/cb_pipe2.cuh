@@ -183,6 +183,9 @@ k_stage_pipe2(Src src, PhysT<T> p, T rka) {
   constexpr int Np = C::Np, Nfp = C::Nfp, NF = C::NFACE, EPB = C::EPB, SP = C::SLOTS;
   constexpr int MJI = DIM * DIM + 1, GC = DIM * DIM + 2 + DIM - 1;
   constexpr int FS = EPB * Nfp, RS = PP::RS, NR = PP::NR, GS = PP::GS;
+  // 3-D N=5 and 6 FP64, 7 to 14 warps per SM: the loads of the heights (gravity)
+  // are started before the wait for the slabs
+  constexpr bool HT = !AFF && sizeof(T) == 8 && DIM == 3 && C::NPT == 1 && C::FPT == 1;
   constexpr size_t TSTRIDE = PP::pad16(PP::TBYTES) / sizeof(T);
   constexpr size_t SSTRIDE = PP::pad16(PP::SBYTES) / sizeof(T);
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -348,6 +351,26 @@ k_stage_pipe2(Src src, PhysT<T> p, T rka) {
       }
     }
 
+    // ---- heights (HT: in flight while the slabs are waited for)
+    T hN[HT ? C::NPT : 1], hM[HT ? C::FPT : 1], hP[HT ? C::FPT : 1];
+    if constexpr (HT) {
+      const T *hg = src.vgeo(it) + Np * GC;
+      if (p.grav != T(0)) {
+#pragma unroll
+        for (int u = 0; u < C::NPT; ++u) {
+          const int slot = tid + u * C::THREADS, el = slot / Np;
+          hN[u] = slot < SP && el < nv ? hg[slot % Np + Np * NVG * (e0 + el)] : T(0);
+        }
+#pragma unroll
+        for (int u = 0; u < C::FPT; ++u) {
+          const int fs = tid + u * C::THREADS, fn = fs % Nfp;
+          const int el = fs / (NF * Nfp), f = (fs / Nfp) % NF;
+          hM[u] = fs < C::FSLOTS && el < nv ? hg[face_node<DIM, Nq>(f, fn) + Np * NVG * (e0 + el)] : T(0);
+          hP[u] = nbv[u] >= 0 ? hg[face_node<DIM, Nq>(nbv[u] & 7, fn) + Np * NVG * (int64_t)(nbv[u] >> 3)] : T(0);
+        }
+      }
+    }
+
     // ---- wait for S[sb] (state + metric) and T[tb] (carry + sgeo)
     if (!mbar_wait_bounded(&barS[sb], (uint32_t)((it / PP::NSB) & 1), src.wait_limit())) timed_out = true;
     if (!mbar_wait_bounded(&barT[tb], (uint32_t)((it / PP::NTB) & 1), src.wait_limit())) timed_out = true;
@@ -400,7 +423,7 @@ k_stage_pipe2(Src src, PhysT<T> p, T rka) {
             for (int c = 0; c < DIM; ++c) met[r][c] = G[(r + DIM * c) * Np + n];
           MJ = G[DIM * DIM * Np + n];
           mji[u] = G[MJI * Np + n];
-          gc = p.grav != T(0) ? vgeo[n + Np * (GC + NVG * (e0 + el))] : T(0);
+          gc = p.grav == T(0) ? T(0) : HT ? hN[HT ? u : 0] : vgeo[n + Np * (GC + NVG * (e0 + el))];
         }
         const T ri = T(1) / q[IR];
         const T P = pressure_ri<DIM, T>(q, ri, gc, p);
@@ -439,7 +462,7 @@ k_stage_pipe2(Src src, PhysT<T> p, T rka) {
         T qM[NS], qq[NS];
 #pragma unroll
         for (int s = 0; s < NS; ++s) qM[s] = Sq[(el * NS + s) * Np + vM] + qr[s];
-        const T gM = (!AFF && p.grav != T(0)) ? vgeo[vM + Np * (GC + NVG * (e0 + el))] : T(0);
+        const T gM = AFF || p.grav == T(0) ? T(0) : HT ? hM[HT ? u : 0] : vgeo[vM + Np * (GC + NVG * (e0 + el))];
         const T riM = T(1) / qM[IR];
         const T PM = pressure_ri<DIM, T>(qM, riM, gM, p);
         T PPv, riP;
@@ -454,7 +477,7 @@ k_stage_pipe2(Src src, PhysT<T> p, T rka) {
           T gP = T(0);
           if (!AFF && p.grav != T(0)) {
             const int64_t e2 = nbv[u] >> 3;
-            gP = vgeo[face_node<DIM, Nq>(nbv[u] & 7, fn) + Np * (GC + NVG * e2)];
+            gP = HT ? hP[HT ? u : 0] : vgeo[face_node<DIM, Nq>(nbv[u] & 7, fn) + Np * (GC + NVG * e2)];
           }
           riP = T(1) / qq[IR];
           PPv = pressure_ri<DIM, T>(qq, riP, gP, p);

@@ -682,7 +682,9 @@ int cb_solver_set_kernel(cb_solver *s, int kernel) {
 
 int cb_solver_get_kernel(const cb_solver *s, int *kernel) {
   if (!s || !kernel) return solver_fail(CB_ERR_ARG, "cb_solver_get_kernel: null argument");
-  const int def = s->prec == 64 ? ops<double>(s)->default_kernel : ops<float>(s)->default_kernel;
+  const bool grav = s->phys.gravity != 0;
+  const int def = s->prec == 64 ? (grav ? ops<double>(s)->gravity_kernel : ops<double>(s)->default_kernel)
+                                : (grav ? ops<float>(s)->gravity_kernel : ops<float>(s)->default_kernel);
   *kernel = s->kernel ? s->kernel : (s->phys.visc > 0 ? 1 : def);
   return CB_OK;
 }
