@@ -43,9 +43,7 @@ struct cb_solver {
   unsigned *status = nullptr;
   double *part = nullptr;
   int part_blocks = 0;
-  cudaGraphExec_t exec = nullptr;       // one step, or two where the state ping-pongs
-  cudaGraphExec_t exec_long = nullptr;  // LONG_REPS times that (see cb_lsrk_run)
-  int64_t reps_run = 0;                 // launches of exec for graph_dt so far
+  cudaGraphExec_t exec = nullptr;  // one step, or two where the state ping-pongs
   double graph_dt = NAN;
   double qref[5] = {0, 0, 0, 0, 0};  // stored state = Q - qref
   int64_t nghost = 0;  // ghost elements after the nelem own ones in Q and the twin
@@ -62,11 +60,6 @@ const double RKA[5] = {0.0, -567301805773.0 / 1357537059087.0, -2404267990393.0 
 const double RKB[5] = {1432997174477.0 / 9575080441755.0, 5161836677717.0 / 13612068292357.0,
                        1720146321549.0 / 2090206949498.0, 3134564353537.0 / 4481467310338.0,
                        2277821191437.0 / 14882151754819.0};
-
-// cb_lsrk_run's long graph: LONG_REPS graphs in one, for states of up to
-// LONG_STATE bytes, after LONG_AFTER of them.
-constexpr int LONG_REPS = 5, LONG_AFTER = 100;
-constexpr int64_t LONG_STATE = 16 << 20;
 
 template <typename T>
 const Ops<T> *ops(const cb_solver *s) {
@@ -151,29 +144,28 @@ cudaError_t enqueue(cb_solver *s, double dt, bool from_user, bool chained) {
 
 void drop_graph(cb_solver *s) {
   if (s->exec) cudaGraphExecDestroy(s->exec);
-  if (s->exec_long) cudaGraphExecDestroy(s->exec_long);
-  s->exec = s->exec_long = nullptr;
-  s->reps_run = 0;
+  s->exec = nullptr;
   s->graph_dt = NAN;
 }
 
-// Graph of `reps` times one step (two where the state ping-pongs).
-int capture(cb_solver *s, double dt, int reps, cudaGraphExec_t *exec) {
+// Graph of one step (two where the state ping-pongs).
+int capture(cb_solver *s, double dt) {
+  drop_graph(s);
   cudaError_t e = cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return solver_fail(CB_ERR_CUDA, "begin capture: %s", cudaGetErrorString(e));
-  cudaError_t e1 = cudaSuccess;
-  for (int r = 0; r < reps && e1 == cudaSuccess; ++r) {
-    e1 = enqueue(s, dt, true, r > 0);
-    if (pingpong(s) && e1 == cudaSuccess) e1 = enqueue(s, dt, false, true);  // two steps
-  }
+  cudaError_t e1 = enqueue(s, dt, true, false);
+  if (pingpong(s) && e1 == cudaSuccess) e1 = enqueue(s, dt, false, true);  // two steps
   cudaGraph_t graph = nullptr;
   e = cudaStreamEndCapture(s->stream, &graph);
   if (e1 == cudaSuccess) e1 = e;
-  if (e1 == cudaSuccess) e1 = cudaGraphInstantiate(exec, graph, 0);
+  if (e1 == cudaSuccess) e1 = cudaGraphInstantiate(&s->exec, graph, 0);
   if (graph) cudaGraphDestroy(graph);
-  if (e1 == cudaSuccess) return CB_OK;
-  *exec = nullptr;
-  return solver_fail(CB_ERR_CUDA, "capture: %s", cudaGetErrorString(e1));
+  if (e1 != cudaSuccess) {
+    s->exec = nullptr;
+    return solver_fail(CB_ERR_CUDA, "capture: %s", cudaGetErrorString(e1));
+  }
+  s->graph_dt = dt;
+  return CB_OK;
 }
 
 int solver_create(cb_solver **out, int dim, int N, int precision, int64_t nelem, int64_t nghost, void *Q,
@@ -575,29 +567,12 @@ int cb_lsrk_run(cb_solver *s, int64_t nsteps, double dt) {
   cudaError_t e;
   if (reps > 0) {
     if (!s->exec || s->graph_dt != dt) {
-      drop_graph(s);
-      const int rc = capture(s, dt, 1, &s->exec);
+      const int rc = capture(s, dt);
       if (rc) return rc;
-      s->graph_dt = dt;
     }
-    // Small meshes: the gap between two graphs (stages in a graph overlap, graphs
-    // do not) costs a good part of a step.  Once a solver has run long enough to
-    // pay for its capture (about 0.3 ms), LONG_REPS graphs are launched as one.
-    // 2-D N=4 10x10 FP64, 20 steps: 137 -> 131 us
-    cudaStreamCaptureStatus outer = cudaStreamCaptureStatusActive;  // (of the caller's own graph)
-    const bool small = per_graph == 2 && state_bytes(s) <= (size_t)LONG_STATE && (s->exec_long ||
-                       (cudaStreamIsCapturing(s->stream, &outer) == cudaSuccess && outer == cudaStreamCaptureStatusNone));
-    for (int64_t r = 0; r < reps;) {
-      if (small && !s->exec_long && s->reps_run + (reps - r) >= LONG_AFTER && reps - r >= LONG_REPS) {
-        const int rc = capture(s, dt, LONG_REPS, &s->exec_long);
-        if (rc) return rc;
-      }
-      const bool lng = s->exec_long && reps - r >= LONG_REPS;
-      if ((e = cudaGraphLaunch(lng ? s->exec_long : s->exec, s->stream)) != cudaSuccess)
+    for (int64_t r = 0; r < reps; ++r)
+      if ((e = cudaGraphLaunch(s->exec, s->stream)) != cudaSuccess)
         return solver_fail(CB_ERR_CUDA, "graph launch: %s", cudaGetErrorString(e));
-      r += lng ? LONG_REPS : 1;
-      s->reps_run += lng ? LONG_REPS : 1;
-    }
   }
   if (rem) {
     if ((e = enqueue(s, dt, true, false)) != cudaSuccess)

@@ -1,6 +1,6 @@
 """Stages of small meshes (geometry and codes loaded before the wait for the
-preceding stage), several steps in one graph, and the per-kernel calls on meshes
-with partial blocks.
+preceding stage), chained launches, and the per-kernel calls on meshes with partial
+blocks.
 
 Tolerances, relative L2 per field: FP64 runs 1e-12, FP32 runs 1e-5, single calls
 1e-13 in FP64 (the bars of the other parity tests); single FP32 calls 1e-5: their
@@ -38,7 +38,7 @@ def solver(m, Q, precision, phys):
 # blocks: N=1 blocks hold 32 elements, N=3 four, N>=5 one; 2-D N=4 ten)
 @pytest.mark.parametrize("precision", [64, 32])
 @pytest.mark.parametrize("N,n", [(1, (3, 3, 3)), (2, (5, 4, 3)), (3, (1, 1, 1)), (3, (8, 8, 9)), (3, (13, 13, 14)),
-                                 (4, (7, 5, 3)), (5, (5, 5, 5)), (6, (3, 4, 3)), (8, (2, 3, 3))])
+                                 (4, (7, 5, 3)), (5, (5, 5, 5)), (6, (3, 4, 3)), (7, (3, 2, 2)), (8, (2, 3, 3))])
 def test_small_stage_3d(N, n, precision):
     m, Q, dt = cube(N, n, True, seed=N)
     phys = dict(dg.WORKLOAD_PHYS, gravity=0.3)
@@ -62,20 +62,18 @@ def test_small_stage_2d(N, side, precision):
     s.close()
 
 
-def test_several_steps_in_one_graph():
-    """A solver that has run 200 steps launches ten steps as one graph: the same
-    kernels in the same order, so the same bits as calls of four steps, which never
-    do; and a new time step starts over."""
-    m, Q = vortex_case(4, 10)
-    a, b = (solver(m, Q, 64, dg.WORKLOAD_PHYS) for _ in range(2))
-    for dt, steps in ((0.002, 300), (0.001, 37), (0.001, 230), (0.002, 24)):
-        a.run(steps, dt)
-        done = 0
-        while done < steps:
-            k = min(4, steps - done)
-            b.run(k, dt)
-            done += k
-        assert np.array_equal(a.state(), b.state()), (dt, steps)
+@pytest.mark.parametrize("dim,N,side,precision", [(2, 4, 10, 64), (2, 7, 30, 32), (3, 3, 8, 32), (3, 4, 9, 64),
+                                                  (3, 6, 5, 64), (3, 7, 6, 64), (3, 8, 5, 64)])
+def test_chained_launches(dim, N, side, precision):
+    """In a graph a stage is launched while the one before it finishes; a single
+    step is launched directly, its first stage after all earlier work.  The same
+    kernels on the same data: the same bits."""
+    m, Q, dt = cube(N, (side,) * 3, True, seed=N) if dim == 3 else (*vortex_case(N, side), 1e-4)
+    a, b = (solver(m, Q, precision, dg.WORKLOAD_PHYS) for _ in range(2))
+    a.run(20, dt)
+    for _ in range(20):
+        b.run(1, dt)
+    assert np.array_equal(a.state(), b.state())
     a.close()
     b.close()
 
