@@ -177,11 +177,6 @@ __device__ __forceinline__ void visc_normal(const T (*g)[3], const T *vel, const
   t[3] = vel[0] * t[0] + vel[1] * t[1] + vel[2] * t[2] + p.cpPr * (g[3][0] * n[0] + g[3][1] * n[1] + g[3][2] * n[2]);
 }
 
-// The gradient of a node is stored as one record of 12 values, ∂_c of u, v, w, T
-// for each direction c (the density gradient does not enter the viscous flux):
-// a neighbour's face node is then 48 (FP32) or 96 contiguous bytes instead of
-// twelve lines of which the ξ faces use one value each.
-constexpr int GREC = 12;
 template <typename T>
 __device__ __forceinline__ void load_grad(const T *rec, T (*g)[3]) {
   constexpr int VW = 16 / (int)sizeof(T);
@@ -691,9 +686,61 @@ __global__ void __launch_bounds__(March<Nq, T>::THREADS, March<Nq, T>::blocks_fo
   }
 }
 
+// Density gradient, one element a block: ∂_c ρ = MJI (-Σ_r Dᵀ(MJ ξ_r,c ρ) +
+// Σ_f sMJ n_c (ρ⁻ + ρ⁺)/2), one component after the other.  Not on a step's path:
+// it runs for stage calls and where a packed gradient is asked for.
+template <int Nq, typename T>
+__global__ void __launch_bounds__(256)
+    k_density_grad(const T *__restrict__ Q, T *__restrict__ out, const T *__restrict__ vgeo, const T *__restrict__ sgeo,
+                   const int32_t *__restrict__ nbr, const T *__restrict__ D, T rho_ref) {
+  constexpr int Np = Nq * Nq * Nq, N2 = Nq * Nq, NS = 5, NVG = 14, NSG = 5, IR = 3, MJF = 9, MJIF = 10;
+  __shared__ T Ds[Nq * Nq], h[3][Np];
+  const int64_t e = blockIdx.x;
+  const T *vg = vgeo + e * (Np * NVG), *rho = Q + e * (Np * NS) + Np * IR;
+  for (int t = threadIdx.x; t < Nq * Nq; t += 256) Ds[t] = D[t];
+  auto face = [&](int f, int fn, T own, int c) {
+    const int32_t code = nbr[f + 6 * e];
+    const T *sg = sgeo + NSG * (fn + (int64_t)N2 * (f + 6 * e));
+    const T other =
+        code < 0 ? own : Q[face_node<3, Nq>(code & 7, fn) + Np * (IR + NS * (int64_t)(code >> 3))] + rho_ref;
+    return sg[3] * sg[c] * (T(0.5) * (own + other));
+  };
+  for (int c = 0; c < 3; ++c) {
+    for (int n = threadIdx.x; n < Np; n += 256) {
+      const T v = vg[n + Np * MJF] * (rho[n] + rho_ref);
+#pragma unroll
+      for (int r = 0; r < 3; ++r) h[r][n] = v * vg[n + Np * (r + 3 * c)];
+    }
+    __syncthreads();
+    for (int n = threadIdx.x; n < Np; n += 256) {
+      const int i = n % Nq, j = n / Nq % Nq, k = n / N2;
+      T a = T(0);
+#pragma unroll
+      for (int m = 0; m < Nq; ++m)
+        a -= Ds[m + Nq * i] * h[0][m + Nq * j + N2 * k] + Ds[m + Nq * j] * h[1][i + Nq * m + N2 * k] +
+             Ds[m + Nq * k] * h[2][i + Nq * j + N2 * m];
+      const T own = rho[n] + rho_ref;
+      if (i == 0) a += face(0, j + Nq * k, own, c);
+      if (i == Nq - 1) a += face(1, j + Nq * k, own, c);
+      if (j == 0) a += face(2, i + Nq * k, own, c);
+      if (j == Nq - 1) a += face(3, i + Nq * k, own, c);
+      if (k == 0) a += face(4, i + Nq * j, own, c);
+      if (k == Nq - 1) a += face(5, i + Nq * j, own, c);
+      out[n + Np * (c + 3 * e)] = a * vg[n + Np * MJIF];
+    }
+    __syncthreads();  // h is rewritten
+  }
+}
+
 template <int Nq, typename T>
 struct MarchLaunch {
   using M = March<Nq, T>;
+  static cudaError_t density(const T *Q, T *out, const T *vgeo, const T *sgeo, const int32_t *nbr, const T *D,
+                             int64_t nelem, T rho_ref, cudaStream_t st) {
+    if (nelem == 0) return cudaSuccess;
+    k_density_grad<Nq, T><<<(unsigned)nelem, 256, 0, st>>>(Q, out, vgeo, sgeo, nbr, D, rho_ref);
+    return cudaGetLastError();
+  }
   template <typename K>
   static cudaError_t launch(K kernel, size_t smem, const MarchArgs<T> &a, const PhysT<T> &p, cudaStream_t st,
                             int chained) {
@@ -759,5 +806,17 @@ struct MarchLaunch {
         &MarchLaunch<6, T_>::grad, &MarchLaunch<7, T_>::grad, &MarchLaunch<8, T_>::grad, &MarchLaunch<9, T_>::grad, \
         &MarchLaunch<10, T_>::grad, &MarchLaunch<11, T_>::grad};                                                    \
     return Nq < 2 || Nq > 11 ? cudaErrorInvalidValue : f[Nq - 2](a, p, st, chained);                                \
+  }                                                                                                                 \
+  template <>                                                                                                       \
+  cudaError_t density_gradient<T_>(int Nq, const T_ *Q, T_ *out, const T_ *vgeo, const T_ *sgeo,                    \
+                                   const int32_t *nbr, const T_ *D, int64_t nelem, T_ rho_ref, cudaStream_t st) {   \
+    static cudaError_t (*const f[])(const T_ *, T_ *, const T_ *, const T_ *, const int32_t *, const T_ *, int64_t, \
+                                    T_, cudaStream_t) = {                                                           \
+        &MarchLaunch<2, T_>::density, &MarchLaunch<3, T_>::density, &MarchLaunch<4, T_>::density,                   \
+        &MarchLaunch<5, T_>::density, &MarchLaunch<6, T_>::density, &MarchLaunch<7, T_>::density,                   \
+        &MarchLaunch<8, T_>::density, &MarchLaunch<9, T_>::density, &MarchLaunch<10, T_>::density,                  \
+        &MarchLaunch<11, T_>::density};                                                                             \
+    return Nq < 2 || Nq > 11 ? cudaErrorInvalidValue                                                                \
+                             : f[Nq - 2](Q, out, vgeo, sgeo, nbr, D, nelem, rho_ref, st);                           \
   }                                                                                                                 \
   }

@@ -5,6 +5,11 @@
 
 namespace cb {
 
+// The gradient of a node is one record of 12 values, ∂_c of u, v, w, T for each
+// direction c: a neighbour's face node is then 48 (FP32) or 96 contiguous bytes
+// instead of twelve lines of which the ξ faces use one value each.
+constexpr int GREC = 12;
+
 // One launch: elements ebeg .. eend - 1 (neighbour indices are absolute).
 template <typename T>
 struct MarchArgs {
@@ -13,7 +18,7 @@ struct MarchArgs {
   const T *vgeo, *sgeo;
   const int32_t *nbr;
   const T *D;
-  T *gq;  // gradient (Np, 5, 3, nelem): written by the gradient pass, read by the viscous stage
+  T *gq;  // gradient records [element][Np][GREC]: written by the gradient pass, read by the viscous stage
   int64_t ebeg, eend;
   Offs<T, 5> qref;
   T rka, rkbdt;
@@ -30,5 +35,10 @@ cudaError_t march_volume(int Nq, T *rhs, const T *Q, const T *vgeo, const T *D, 
                          cudaStream_t st);
 template <typename T>
 cudaError_t march_grad(int Nq, const MarchArgs<T> &a, const PhysT<T> &p, cudaStream_t st, int chained);
+// Density gradient (Np, 3, nelem) of the state Q, which the records leave out (it
+// does not enter the viscous flux): for callers who take the whole gradient.
+template <typename T>
+cudaError_t density_gradient(int Nq, const T *Q, T *out, const T *vgeo, const T *sgeo, const int32_t *nbr, const T *D,
+                             int64_t nelem, T rho_ref, cudaStream_t st);
 
 }  // namespace cb

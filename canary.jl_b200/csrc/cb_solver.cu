@@ -20,6 +20,7 @@
 
 #include "../../include/canary_b200.h"
 #include "cb_batch.cuh"
+#include "cb_march.h"
 #include "cb_ops.h"
 
 using namespace cb;
@@ -37,6 +38,13 @@ struct cb_solver {
   const int64_t *vmapM = nullptr, *vmapP = nullptr, *bnd = nullptr;
   int32_t *nbr = nullptr;
   void *gradQ = nullptr, *rhs_gradQ = nullptr;
+  // form the gradient buffer is in: 0 not written yet, 1 (Np, nstate, dim,
+  // elements), 2 records (grad_at)
+  int grad_form = 0;
+  // records: the state (input of the last stage of a run) whose density
+  // gradient the buffer still lacks; no pass reads it, so it is formed when
+  // the gradient is packed
+  const void *rho_src = nullptr;
   cb_phys phys{};
   cudaStream_t stream = nullptr;
   bool own_stream = false;
@@ -186,6 +194,86 @@ cudaError_t settle(cb_solver *s) {
   return cudaMemcpyAsync(s->Q, s->Qalt, state_bytes(s), cudaMemcpyDeviceToDevice, s->stream);
 }
 
+// The column-march passes (3-D) keep the gradient as records (grad_at), the
+// other passes as (Np, nstate, dim, elements): the form of the kernel choice.
+bool records_wanted(const cb_solver *s) {
+  return fused_visc(s) && s->dim == 3 && (s->kernel == 0 || !ns_stage_form(s));
+}
+// the form the buffer is in (one that holds nothing yet is in any form)
+bool records(cb_solver *s) {
+  if (!s->grad_form) s->grad_form = records_wanted(s) ? 2 : 1;
+  return s->grad_form == 2;
+}
+int64_t nodes(const cb_solver *s) {
+  const int64_t Nq = s->N + 1;
+  return s->dim == 2 ? Nq * Nq : Nq * Nq * Nq;
+}
+unsigned blocks_for(int64_t total) { return (unsigned)std::min<int64_t>((total + 255) / 256, 148 * 16); }
+
+// Density gradient of the state `src` into the records' density part.
+template <typename T>
+cudaError_t density_gradient(cb_solver *s, const void *src) {
+  s->rho_src = nullptr;
+  return cb::density_gradient<T>(s->N + 1, (const T *)src, (T *)s->gradQ + GREC * nodes(s) * (s->nelem + s->nghost),
+                                 (const T *)s->vgeo, (const T *)s->sgeo, s->nbr, (const T *)s->D, s->nelem,
+                                 T(s->qref[3]), s->stream);
+}
+cudaError_t density_gradient(cb_solver *s, const void *src) {
+  return s->prec == 64 ? density_gradient<double>(s, src) : density_gradient<float>(s, src);
+}
+// the whole gradient, as far as a run left it
+cudaError_t complete_gradient(cb_solver *s) { return s->rho_src ? density_gradient(s, s->rho_src) : cudaSuccess; }
+
+// Value of gradient component d of field s5 at a node in the records' form of
+// a buffer of `nall` elements: [nall][Np][GREC] for u, v, w and T, then
+// [nall][3][Np] for the density, which no pass reads.
+template <typename T>
+__host__ __device__ __forceinline__ T *grad_at(T *gq, int64_t Np, int64_t nall, int64_t el, int64_t node, int s5, int d) {
+  return s5 == 3 ? gq + GREC * Np * nall + node + Np * (d + 3 * el)
+                 : gq + GREC * (node + Np * el) + 4 * d + (s5 == 4 ? 3 : s5);
+}
+
+// The gradient between its two forms: `plain` is (Np, 5, 3, nall).
+template <typename T>
+__global__ void k_grad_form(bool to_records, T *__restrict__ plain, T *__restrict__ rec, int64_t Np, int64_t nall) {
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < 15 * Np * nall; t += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t el = t / (15 * Np);
+    const int c = (int)(t / Np % 15);
+    T *r = grad_at(rec, Np, nall, el, t % Np, c % 5, c / 5);
+    if (to_records) *r = plain[t];
+    else plain[t] = *r;
+  }
+}
+// Bring the gradient buffer into the form that the kernel choice works with
+// (its values stay: a choice made between two passes changes no result).
+cudaError_t adopt_form(cb_solver *s) {
+  const bool want = records_wanted(s);
+  if (records(s) == want) return cudaSuccess;
+  cudaError_t e = complete_gradient(s);
+  if (e != cudaSuccess) return e;
+  const int64_t Np = nodes(s), nall = s->nelem + s->nghost;
+  const size_t bytes = (s->prec == 64 ? 8 : 4) * (size_t)(15 * Np * nall);
+  void *old = nullptr;
+  if ((e = cudaMallocAsync(&old, bytes, s->stream)) != cudaSuccess) return e;
+  if ((e = cudaMemcpyAsync(old, s->gradQ, bytes, cudaMemcpyDeviceToDevice, s->stream)) == cudaSuccess) {
+    void *plain = want ? old : s->gradQ, *rec = want ? s->gradQ : old;
+    if (s->prec == 64)
+      k_grad_form<double><<<blocks_for(15 * Np * nall), 256, 0, s->stream>>>(want, (double *)plain, (double *)rec, Np, nall);
+    else
+      k_grad_form<float><<<blocks_for(15 * Np * nall), 256, 0, s->stream>>>(want, (float *)plain, (float *)rec, Np, nall);
+    if ((e = cudaGetLastError()) == cudaSuccess) s->grad_form = want ? 2 : 1;
+  }
+  const cudaError_t ef = cudaFreeAsync(old, s->stream);
+  return e == cudaSuccess ? ef : e;
+}
+// The same before a gradient pass, which writes every own element.
+cudaError_t adopt_form_anew(cb_solver *s) {
+  if (s->nghost) return adopt_form(s);
+  s->grad_form = records_wanted(s) ? 2 : 1;
+  s->rho_src = nullptr;
+  return cudaSuccess;
+}
+
 // one pass of an RK stage: pass 0 the viscous gradient of the current state
 // (nothing for the inviscid form), pass 1 the stage from the current buffer
 // into the other
@@ -207,9 +295,14 @@ cudaError_t enqueue_pass(cb_solver *s, int st, double dt, int pass) {
     I.status = visc_status(s);
     I.dt = dt;
     for (int k = 0; k < 5; ++k) I.qref[k] = T(s->qref[k]);
-    return pass == 0 ? o->ns_pass(0, I, (T *)s->gradQ, s->nelem, p, T(0), T(0), s->stream, s->kernel, 0)
-                     : o->ns_pass(1, I, (T *)s->gradQ, s->nelem, p, T(RKA[(st + 1) % 5]), T(RKB[st] * dt), s->stream,
-                                  s->kernel, 0);
+    cudaError_t e = pass == 0 ? adopt_form_anew(s) : adopt_form(s);
+    if (e != cudaSuccess) return e;
+    if (pass == 0) {
+      e = o->ns_pass(0, I, (T *)s->gradQ, s->nelem, p, T(0), T(0), s->stream, s->kernel, 0);
+      return e == cudaSuccess && records(s) ? density_gradient(s, a) : e;
+    }
+    if ((e = complete_gradient(s)) != cudaSuccess) return e;  // the stage may overwrite rho_src
+    return o->ns_pass(1, I, (T *)s->gradQ, s->nelem, p, T(RKA[(st + 1) % 5]), T(RKB[st] * dt), s->stream, s->kernel, 0);
   }
   if (pass == 0) return cudaSuccess;
   Offs<T, 5> q5;
@@ -218,17 +311,58 @@ cudaError_t enqueue_pass(cb_solver *s, int st, double dt, int pass) {
                     p, q5, T(RKA[(st + 1) % 5]), T(RKB[st] * dt), s->status, s->stream, 0, s->kernel, 0, 0);
 }
 
-// The column-march passes (3-D) keep the gradient as records of 12 values per
-// node (cb_march.cuh), the other passes as (Np, nstate, dim, nelem).
-bool grad_records(const cb_solver *s) { return fused_visc(s) && s->dim == 3 && (s->kernel == 0 || !ns_stage_form(s)); }
-
 // Copy whole elements: gather `n` elements listed in `idx` (device int64) of
-// `src` (ew values each) into `dst`, one every `dw` values.
+// `src` (ew values each) into the contiguous `dst`.
 template <typename T>
 __global__ void k_pack(const T *__restrict__ src, const int64_t *__restrict__ idx, int64_t n, int64_t ew,
-                       int64_t dw, T *__restrict__ dst) {
+                       T *__restrict__ dst) {
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n * ew; t += (int64_t)gridDim.x * blockDim.x)
-    dst[t / ew * dw + t % ew] = src[idx[t / ew] * ew + t % ew];
+    dst[t] = src[idx[t / ew] * ew + t % ew];
+}
+
+// Whole elements of a gradient kept as records, between the buffer and `buf`
+// (n elements of (Np, 5, 3)): elements idx[0..n) (pack), or `first` and on.
+template <typename T>
+__global__ void k_grad_elems(bool pack, T *__restrict__ gq, const int64_t *__restrict__ idx, int64_t first, int64_t n,
+                             int64_t Np, int64_t nall, T *__restrict__ buf) {
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < 15 * Np * n; t += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t i = t / (15 * Np);
+    const int c = (int)(t / Np % 15);
+    T *r = grad_at(gq, Np, nall, idx ? idx[i] : first + i, t % Np, c % 5, c / 5);
+    if (pack) buf[t] = *r;
+    else *r = buf[t];
+  }
+}
+cudaError_t grad_elems(cb_solver *s, bool pack, const int64_t *idx, int64_t first, int64_t n, void *buf) {
+  const int64_t Np = nodes(s), nall = s->nelem + s->nghost;
+  const unsigned grid = blocks_for(15 * Np * n);
+  if (s->prec == 64)
+    k_grad_elems<double><<<grid, 256, 0, s->stream>>>(pack, (double *)s->gradQ, idx, first, n, Np, nall, (double *)buf);
+  else
+    k_grad_elems<float><<<grid, 256, 0, s->stream>>>(pack, (float *)s->gradQ, idx, first, n, Np, nall, (float *)buf);
+  return cudaGetLastError();
+}
+
+// After an odd number of steps of a run whose gradient is kept as records: the
+// state goes back from the twin into Q, and the density of Q, which the last
+// stage read, into the twin (see rho_src).
+template <typename T, typename I>
+__global__ void k_copy_back(T *__restrict__ Q, T *__restrict__ twin, I Np, I total) {
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
+    const T v = twin[t];
+    if ((I)t / Np % 5 == 3) twin[t] = Q[t];
+    Q[t] = v;
+  }
+}
+template <typename T>
+cudaError_t copy_back(cb_solver *s) {
+  const int64_t Np = nodes(s), total = Np * 5 * s->nelem;
+  const unsigned grid = blocks_for(total);
+  if (total <= 0xffffffffll)
+    k_copy_back<T, uint32_t><<<grid, 256, 0, s->stream>>>((T *)s->Q, (T *)s->Qalt, (uint32_t)Np, (uint32_t)total);
+  else
+    k_copy_back<T, int64_t><<<grid, 256, 0, s->stream>>>((T *)s->Q, (T *)s->Qalt, Np, total);
+  return cudaGetLastError();
 }
 
 // Face traces of a partitioned solve.  Entry i of `codes` is (element << 3) |
@@ -237,8 +371,8 @@ __global__ void k_pack(const T *__restrict__ src, const int64_t *__restrict__ id
 // component at element offset Np·c.  Pack reads own elements (0 .. nown - 1)
 // into buf[(i·W + c)·Nfp + fn]; unpack writes ghost slots (element nown + g
 // for code g << 3 | face).  rec: the gradient as records (component c is
-// direction c / 5 of field c % 5; the density gradient is not kept, its
-// entries are 0).  An entry out of range is skipped and raises ST_MESH.
+// direction c / 5 of field c % 5).  An entry out of range is skipped and
+// raises ST_MESH.
 template <int DIM, typename T>
 __global__ void k_faces(bool pack, bool rec, T *__restrict__ arr, const int64_t *__restrict__ codes, int64_t n, int Nq,
                         int W, int64_t nown, int64_t nghost, T *__restrict__ buf, unsigned *status) {
@@ -255,22 +389,20 @@ __global__ void k_faces(bool pack, bool rec, T *__restrict__ arr, const int64_t 
     }
     const int64_t el = pack ? e : nown + e;
     const int64_t node = face_node_rt<DIM>(Nq, f, fn);
-    if (rec && c % 5 == 3) {
-      if (pack) buf[t] = T(0);
-      continue;
-    }
-    T *a = rec ? arr + 12 * (node + Np * el) + 4 * (c / 5) + (c % 5 == 4 ? 3 : c % 5) : arr + node + (int64_t)Np * (c + (int64_t)W * el);
+    T *a = rec ? grad_at(arr, Np, nown + nghost, el, node, c % 5, c / 5) : arr + node + (int64_t)Np * (c + (int64_t)W * el);
     if (pack) buf[t] = *a;
     else *a = buf[t];
   }
 }
 
 template <typename T>
-cudaError_t launch_faces(const cb_solver *s, bool pack, int what, const int64_t *codes, int64_t n, void *buf) {
+cudaError_t launch_faces(cb_solver *s, bool pack, int what, const int64_t *codes, int64_t n, void *buf) {
   const int Nq = s->N + 1, Nfp = s->dim == 2 ? Nq : Nq * Nq;
   const int W = (s->dim == 2 ? 4 : 5) * (what ? s->dim : 1);
   T *arr = (T *)(what ? s->gradQ : (s->cur ? s->Qalt : s->Q));
-  const bool rec = what && grad_records(s);
+  const bool rec = what && records(s);
+  const cudaError_t e = what ? complete_gradient(s) : cudaSuccess;
+  if (e != cudaSuccess) return e;
   const int64_t total = n * W * Nfp;
   const int grid = (int)std::min<int64_t>((total + 255) / 256, 148 * 16);
   if (s->dim == 2)
@@ -406,17 +538,19 @@ int cb_solver_pack(cb_solver *s, int what, const int64_t *elems, int64_t n, void
   if (!s || n < 0 || (n && (!elems || !buf)) || what < 0 || what > 1 || (what == 1 && !s->gradQ))
     return solver_fail(CB_ERR_ARG, "cb_solver_pack: bad arguments");
   if (!n) return CB_OK;
-  const int Nq = s->N + 1;
-  const int64_t Np = s->dim == 2 ? (int64_t)Nq * Nq : (int64_t)Nq * Nq * Nq;
-  const int64_t dw = Np * (s->dim == 2 ? 4 : 5) * (what ? s->dim : 1);
-  const int64_t ew = what && grad_records(s) ? 12 * Np : dw;
-  const int grid = (int)std::min<int64_t>((n * ew + 255) / 256, 148 * 16);
-  const void *src = what ? s->gradQ : (s->cur ? s->Qalt : s->Q);
-  if (s->prec == 64)
-    k_pack<double><<<grid, 256, 0, s->stream>>>((const double *)src, elems, n, ew, dw, (double *)buf);
-  else
-    k_pack<float><<<grid, 256, 0, s->stream>>>((const float *)src, elems, n, ew, dw, (float *)buf);
-  const cudaError_t e = cudaGetLastError();
+  cudaError_t e = what ? complete_gradient(s) : cudaSuccess;
+  if (e == cudaSuccess && what && records(s)) {
+    e = grad_elems(s, true, elems, 0, n, buf);
+  } else if (e == cudaSuccess) {
+    const int64_t ew = nodes(s) * (s->dim == 2 ? 4 : 5) * (what ? s->dim : 1);
+    const unsigned grid = blocks_for(n * ew);
+    const void *src = what ? s->gradQ : (s->cur ? s->Qalt : s->Q);
+    if (s->prec == 64)
+      k_pack<double><<<grid, 256, 0, s->stream>>>((const double *)src, elems, n, ew, (double *)buf);
+    else
+      k_pack<float><<<grid, 256, 0, s->stream>>>((const float *)src, elems, n, ew, (float *)buf);
+    e = cudaGetLastError();
+  }
   return e == cudaSuccess ? CB_OK : solver_fail(CB_ERR_CUDA, "cb_solver_pack: %s", cudaGetErrorString(e));
 }
 
@@ -426,10 +560,14 @@ int cb_solver_unpack(cb_solver *s, int what, const void *buf, int64_t first, int
   if (first < 0 || n < 0 || first + n > s->nghost || (n && !buf))
     return solver_fail(CB_ERR_ARG, "cb_solver_unpack: ghost range outside 0..%lld", (long long)s->nghost);
   if (!n) return CB_OK;
-  const size_t sw = state_bytes(s) / (size_t)s->nelem * (what ? s->dim : 1);  // bytes per element in buf
-  const size_t ew = what && grad_records(s) ? sw / 15 * 12 : sw;
-  char *dst = (char *)(what ? s->gradQ : (s->cur ? s->Qalt : s->Q)) + ew * (size_t)(s->nelem + first);
-  const cudaError_t e = cudaMemcpy2DAsync(dst, ew, buf, sw, ew, (size_t)n, cudaMemcpyDeviceToDevice, s->stream);
+  cudaError_t e;
+  if (what && records(s)) {
+    e = grad_elems(s, false, nullptr, s->nelem + first, n, const_cast<void *>(buf));
+  } else {
+    const size_t ew = state_bytes(s) / (size_t)s->nelem * (what ? s->dim : 1);
+    char *dst = (char *)(what ? s->gradQ : (s->cur ? s->Qalt : s->Q)) + ew * (size_t)(s->nelem + first);
+    e = cudaMemcpyAsync(dst, buf, ew * (size_t)n, cudaMemcpyDeviceToDevice, s->stream);
+  }
   return e == cudaSuccess ? CB_OK : solver_fail(CB_ERR_CUDA, "cb_solver_unpack: %s", cudaGetErrorString(e));
 }
 
@@ -562,6 +700,9 @@ int cb_lsrk_run(cb_solver *s, int64_t nsteps, double dt) {
   if (nsteps == 0) return CB_OK;
   cudaError_t e0 = settle(s);  // a state left in the twin by the stage API
   if (e0 != cudaSuccess) return solver_fail(CB_ERR_CUDA, "state copy: %s", cudaGetErrorString(e0));
+  if (s->phys.visc > 0 && (e0 = adopt_form_anew(s)) != cudaSuccess)
+    return solver_fail(CB_ERR_CUDA, "gradient form: %s", cudaGetErrorString(e0));
+  const bool rec = records_wanted(s);
   const int64_t per_graph = pingpong(s) ? 2 : 1;
   const int64_t reps = nsteps / per_graph, rem = nsteps % per_graph;
   cudaError_t e;
@@ -577,12 +718,19 @@ int cb_lsrk_run(cb_solver *s, int64_t nsteps, double dt) {
   if (rem) {
     if ((e = enqueue(s, dt, true, false)) != cudaSuccess)
       return solver_fail(CB_ERR_CUDA, "step launch: %s", cudaGetErrorString(e));
-    const int Nq = s->N + 1;
-    const int64_t Np = s->dim == 2 ? (int64_t)Nq * Nq : (int64_t)Nq * Nq * Nq;
-    const size_t bytes = (s->prec == 64 ? 8 : 4) * (size_t)Np * (s->dim == 2 ? 4 : 5) * s->nelem;
-    if ((e = cudaMemcpyAsync(s->Q, s->Qalt, bytes, cudaMemcpyDeviceToDevice, s->stream)) != cudaSuccess)
-      return solver_fail(CB_ERR_CUDA, "state copy: %s", cudaGetErrorString(e));
   }
+  // records: the density gradient is left to whoever packs it, where the last
+  // stage's input stays in the twin until then
+  const void *last = rem ? s->Q : s->Qalt;
+  if (rec && s->nghost && (e = density_gradient(s, last)) != cudaSuccess)
+    return solver_fail(CB_ERR_CUDA, "density gradient: %s", cudaGetErrorString(e));
+  if (rec && !s->nghost) s->rho_src = s->Qalt;
+  if (rem && rec && !s->nghost) {
+    e = s->prec == 64 ? copy_back<double>(s) : copy_back<float>(s);
+  } else if (rem) {
+    e = cudaMemcpyAsync(s->Q, s->Qalt, state_bytes(s), cudaMemcpyDeviceToDevice, s->stream);
+  }
+  if (rem && e != cudaSuccess) return solver_fail(CB_ERR_CUDA, "state copy: %s", cudaGetErrorString(e));
   return CB_OK;
 }
 
@@ -632,6 +780,8 @@ int cb_solver_set_offset(cb_solver *s, const double *qref) {
         return solver_fail(CB_ERR_UNSUPPORTED, "state offsets: the viscous form of this order has none");
     return CB_OK;
   }
+  const cudaError_t e = complete_gradient(s);  // (of the state with its old offset)
+  if (e != cudaSuccess) return solver_fail(CB_ERR_CUDA, "cb_solver_set_offset: %s", cudaGetErrorString(e));
   for (int k = 0; k < (s->dim == 2 ? 4 : 5); ++k) s->qref[k] = qref[k];
   drop_graph(s);
   return CB_OK;

@@ -225,6 +225,8 @@ int cb_solver_destroy(cb_solver *s);
  * form (the orders with fused passes) also exchanges the gradient (what = 1)
  * between the stage's gradient pass and its stage pass
  * (cb_solver_stage_pass, pass 0 then 1); cb_solver_stage runs both passes.
+ * Elements travel as (Np, nstate) values of the state and (Np, nstate, dim) of
+ * the gradient, whatever kernels the ranks run.
  * A stage goes from the current state into the other buffer and returns the
  * new current buffer; cb_solver_settle copies a state left in the twin back
  * into Q (cb_lsrk_run and cb_solver_sums handle it themselves). */
