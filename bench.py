@@ -62,7 +62,7 @@ def bytes_per_node(dim, N, w):
 
 
 L2_BYTES = 126e6
-STAGE_KERNELS = {1: "k_stage_pipe2", 2: "k_stage_mma", 3: "k_stage", 4: "k_stage_lean"}
+STAGE_KERNELS = {1: "k_stage_pipe2", 2: "k_stage_mma", 3: "k_stage", 4: "k_stage_lean", 5: "k_march_stage"}
 
 
 def measured_peaks():

@@ -438,18 +438,19 @@ class LSRK:
         check(_lib.lib().cb_solver_status_async(self._h, C.c_void_p(host.data_ptr())))
 
     def set_kernel(self, kernel: int) -> None:
-        """Stage kernel: 0 = the shape's default (viscous 3-D: the grid-line
-        passes), 1 = the CUDA-core stages (viscous: the pipelined passes),
+        """Stage kernel: 0 = the mesh's default, 1 = the CUDA-core stages
+        (viscous: the pipelined passes),
         2 = the tensor-core (DMMA) stage of the inviscid 3-D N=7 form, 3 = the
         unpipelined grouped stages (for the fused viscous form: the grouped
         passes instead of the pipelined ones), 4 = the lean pipelined stage
-        of the inviscid form (only the state staged in shared memory)."""
+        of the inviscid form (only the state staged in shared memory), 5 = the
+        grid-line stages (inviscid 3-D N=10 and FP64 N=8, 9; viscous 3-D)."""
         check(_lib.lib().cb_solver_set_kernel(self._h, int(kernel)))
 
     @property
     def kernel(self) -> int:
         """The stage kernel the solver runs: 1 CUDA-core, 2 tensor-core, 3
-        grouped, 4 lean."""
+        grouped, 4 lean, 5 grid lines."""
         v = C.c_int(0)
         check(_lib.lib().cb_solver_get_kernel(self._h, C.byref(v)))
         return v.value

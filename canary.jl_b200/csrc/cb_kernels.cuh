@@ -930,8 +930,7 @@ struct Launch {
   // Whether the lean pipelined stage is built for this shape, and whether it
   // is the shape's default (where the tensor-core stage is not).
   static constexpr bool LEAN_OK = Lean<DIM, Nq, T>::OK;
-  // Whether the unpipelined choice (3) and the default are the column march
-  // (cb_march.cuh) instead of the grouped stage: where the all-at-once plan
+  // Whether the default is the column march (cb_march.cuh): where the all-at-once plan
   // leaves one block per SM (B200, one mesh of 5.8-6.5 M nodes, ms per step:
   // N=10 FP64 4.28 -> 3.35, FP32 1.92 -> 1.61; N=9 FP64 2.96 -> 2.72; N=8 FP64
   // 16^3 1.58 -> 1.43, under gravity 1.64 -> 1.45).  Below,
@@ -950,7 +949,7 @@ struct Launch {
   // 3.18 / 3.42, FP32 1.83 / 1.33 / 1.64; N=1: FP64 4.52 / 3.30 / 3.90, FP32
   // 2.87 / 1.36 / 2.43.  3-D N=7 runs the tensor-core stage in both precisions.
   static constexpr int DEFAULT_KERNEL =
-      MARCH         ? 3
+      MARCH         ? 5
       : MMA_DEFAULT ? 2
       : DIM == 3 && sizeof(T) == 8 && LEAN_OK && (Nq == 4 || Nq == 5) ? 4
       : DIM == 3 && (Nq <= 3 || (sizeof(T) == 4 && Nq <= 10)) ? 3
@@ -962,13 +961,22 @@ struct Launch {
   static constexpr int GRAVITY_KERNEL = DIM == 3 && sizeof(T) == 8 && Nq == 7   ? 4
                                         : DIM == 3 && sizeof(T) == 8 && Nq == 5 ? 3
                                                                                 : DEFAULT_KERNEL;
-  // Small launches of the shapes that default to the grouped stage, and of 2-D,
-  // run its EARLY form: up to EARLY_BLOCKS blocks per SM.
+  // The grouped stage of small meshes is its EARLY form, and small 2-D meshes
+  // default to it: up to EARLY_BLOCKS blocks per SM.
   static constexpr bool EARLY_OK = C::NPT == 1 && !MARCH && (DIM == 2 || DEFAULT_KERNEL == 3);
   // (us a stage, stages in a row on one solver: FP32 3-D N=3 8^3 4.9 -> 3.0, 12^3
   // 6.4 -> 5.6, N=4 8^3 5.9 -> 4.4, N=6 6^3 6.8 -> 5.3, 2-D N=4 48^2 5.7 -> 3.2;
   // FP64 2-D N=4 10^2 4.9 -> 2.9, but N=7 32^2 4.5 at one block, 5.6 at two)
   static constexpr int EARLY_BLOCKS = sizeof(T) == 4 ? 4 : 1;
+  static bool small_mesh(int64_t nelem) {
+    return EARLY_OK && (nelem + C::EPB - 1) / C::EPB <= (int64_t)EARLY_BLOCKS * num_sms();
+  }
+  // The stage kernel that choice 0 resolves to on a mesh of nelem elements.
+  static int choice(int64_t nelem, bool gravity) {
+    if (MARCH) return 5;
+    if (DIM == 2 && small_mesh(nelem)) return 3;
+    return gravity ? GRAVITY_KERNEL : DEFAULT_KERNEL;
+  }
   // Resident blocks per SM of a kernel at `smem` bytes, from the occupancy
   // calculator, cached per device in `cache`.
   template <typename K>
@@ -988,50 +996,57 @@ struct Launch {
     *out = cache[dev];
     return cudaSuccess;
   }
-  // kernel: 0 = the default for the shape (DEFAULT_KERNEL), 1 = the
-  // CUDA-core stages only, 2 = the tensor-core stage (cudaErrorNotSupported
-  // where it is not built), 3 = the unpipelined grouped stage k_stage, 4 =
-  // the lean pipelined stage k_stage_lean (state-only staging; the pipelined
-  // stage where the arrays are not 16-byte aligned).  probe != 0: the timeout
-  // test hook of the pipelined, lean and tensor-core stages (see MeshSrc);
-  // shapes without one return cudaErrorNotSupported for it.
+  // kernel: 0 = the default for the mesh (choice), 1 = the CUDA-core stages
+  // only, 2 = the tensor-core stage (cudaErrorNotSupported where it is not
+  // built), 3 = the unpipelined grouped stage k_stage, 4 = the lean pipelined
+  // stage k_stage_lean (state-only staging; the pipelined stage where the
+  // arrays are not 16-byte aligned), 5 = the column march (where it is the
+  // default).  probe != 0: the timeout test hook of the pipelined, lean and
+  // tensor-core stages (see MeshSrc); shapes without one return
+  // cudaErrorNotSupported for it.
   // ebeg: the launch covers elements ebeg .. nelem - 1 (neighbour indices
-  // stay absolute); only the pipelined, lean and tensor-core stages and the
-  // default column march and grouped stage take ebeg > 0, the others return cudaErrorNotSupported for it.  chained: the
-  // stream's preceding launch is a stage of the same solve (see grid_wait).
+  // stay absolute); only the pipelined, lean and tensor-core stages, the march
+  // and the default grouped stage take ebeg > 0, the others return
+  // cudaErrorNotSupported for it.  nall: elements of the whole mesh, by which
+  // the default is chosen: a stage in parts runs the kernel of the stage in one
+  // call.  chained: the stream's preceding launch is a stage of the same solve
+  // (see grid_wait).
   static cudaError_t stage(const T *Qin, T *Qout, T *rhs, const T *vgeo, const T *sgeo,
                            const int32_t *nbr, const T *D, int64_t nelem, const PhysT<T> &p,
                            const Offs<T, NS> &qref, T rka, T rkbdt, unsigned *status,
-                           cudaStream_t st, int probe = 0, int kernel = 0, int64_t ebeg = 0, int chained = 0) {
+                           cudaStream_t st, int probe, int kernel, int64_t ebeg, int chained, int64_t nall) {
     constexpr bool pipe_ok = Pipe<DIM, Nq, T>::OK;
+    static_assert(Pipe2<DIM, Nq, T>::OK || (DEFAULT_KERNEL != 1 && GRAVITY_KERNEL != 1),
+                  "choice 1 as the default takes element ranges");
     const bool aligned = ((reinterpret_cast<uintptr_t>(Qin) | reinterpret_cast<uintptr_t>(vgeo)) & 15) == 0;
     const bool aligned2 = aligned && ((reinterpret_cast<uintptr_t>(rhs) | reinterpret_cast<uintptr_t>(sgeo)) & 15) == 0;
     if (ebeg < 0 || ebeg > nelem) return cudaErrorInvalidValue;
+    const bool by_default = kernel == 0 || (kernel == 5 && probe);
+    if (by_default) {
+      // the grouped stage and the march take no test hook: that call takes the
+      // pipelined stage, or the lean one where the pipelined plan does not fit
+      // shared memory (3-D N=9 FP64, N=10 FP32)
+      kernel = !probe                                             ? choice(nall, p.grav != T(0))
+               : DEFAULT_KERNEL == 2 || DEFAULT_KERNEL == 4        ? DEFAULT_KERNEL
+               : Pipe2<DIM, Nq, T>::OK || !LEAN_OK                 ? 1
+                                                                   : 4;
+      if (kernel == 2 && !aligned2) kernel = 1;
+    }
     if constexpr (MARCH) {
-      if (!probe && (kernel == 0 || (kernel == 3 && !ebeg))) {
+      if (kernel == 5) {
         MarchArgs<T> a{Qin, Qout, rhs, vgeo, sgeo, nbr, D, nullptr, ebeg, nelem, {}, rka, rkbdt, status};
         for (int s = 0; s < NS; ++s) a.qref.v[s] = qref.v[s];
         return march_stage<T>(Nq, false, a, p, st, chained);
       }
     }
-    // the shape's default; the grouped stage takes no test hook: that call
-    // takes the pipelined stage, or the lean one where the pipelined plan does
-    // not fit shared memory (3-D N=10 FP32)
-    const int dflt = p.grav != T(0) && !probe ? GRAVITY_KERNEL : DEFAULT_KERNEL;
-    const bool grouped_default = kernel == 0 && dflt == 3 && !probe;
-    if (kernel == 0 && (probe || ebeg) && !grouped_default && (DEFAULT_KERNEL == 1 || DEFAULT_KERNEL == 3))
-      kernel = (Pipe2<DIM, Nq, T>::OK || !LEAN_OK) ? 1 : 4;
-    else if (grouped_default)
-      kernel = 3;
-    else if (kernel == 0 && dflt == 4)
-      kernel = 4;
-    if (kernel == 2 && !(MMA_OK && aligned2)) return cudaErrorNotSupported;
+    if (kernel == 5 || (kernel == 2 && !(MMA_OK && aligned2))) return cudaErrorNotSupported;
+    if (kernel == 3 && (probe || (ebeg && !by_default))) return cudaErrorNotSupported;
     if (kernel == 4 && !LEAN_OK) return cudaErrorNotSupported;
     if (kernel == 4 && !aligned2) kernel = 1;  // bulk copies need 16-byte aligned slabs
     const int64_t groups = (nelem - ebeg + C::EPB - 1) / C::EPB;
     if (groups == 0) return cudaSuccess;
     if constexpr (EARLY_OK) {
-      if ((grouped_default || (DIM == 2 && kernel == 0 && !probe && !ebeg)) && groups <= EARLY_BLOCKS * num_sms()) {
+      if (kernel == 3 && small_mesh(nall)) {
         const size_t sm = smem_stage();
         const cudaError_t err = prep(k_stage<DIM, Nq, T, true>, sm);
         if (err != cudaSuccess) return err;
@@ -1040,7 +1055,7 @@ struct Launch {
       }
     }
     if constexpr (MMA_OK) {
-      if ((kernel == 2 || (kernel == 0 && MMA_DEFAULT)) && aligned2) {
+      if (kernel == 2) {
         using S = MeshSrc<T, NS, C::EPB>;  // MeshSrc<T, 5, 1> here
         using PM = PipeMT<T>;
         static int per_sm[MAX_DEVICES] = {0};
@@ -1079,7 +1094,7 @@ struct Launch {
       if (g > groups) g = groups;
       const S src{Qin, Qout, rhs, vgeo, sgeo, nbr, D, nelem, qref, rkbdt, status, probe, ebeg};
       return launch_stage_kernel(k_stage_pipe2<DIM, Nq, T, S>, (unsigned)g, C::THREADS, sm, st, chained, src, p, rka);
-    } else if (probe || (ebeg && !grouped_default)) {
+    } else if (probe || (ebeg && kernel != 3)) {
       return cudaErrorNotSupported;
     } else if (pipe_ok && aligned && kernel != 3) {
       using PP = Pipe<DIM, Nq, T>;

@@ -23,20 +23,23 @@ struct Ops {
   // the stage with, after the stream: the timeout test hook flag (each
   // block's first state copy withheld and a short wait limit;
   // cudaErrorNotSupported where no pipelined stage runs), the kernel choice
-  // (0 the shape's default, 1 the CUDA-core stages, 2 the tensor-core stage;
-  // cudaErrorNotSupported where the choice is not built) and the first
-  // element of the launch (elements first .. nelem - 1), and whether the
-  // stream's preceding launch is a stage of the same solve (see grid_wait)
+  // (0 the mesh's default, 1 the CUDA-core stages, 2 the tensor-core stage and
+  // so on, see Launch::stage; cudaErrorNotSupported where the choice is not
+  // built) and the first element of the launch (elements first .. nelem - 1),
+  // whether the stream's preceding launch is a stage of the same solve (see
+  // grid_wait) and the elements of the whole mesh
   cudaError_t (*stage_k)(const T *, T *, T *, const T *, const T *, const int32_t *, const T *, int64_t,
-                         const PhysT<T> &, const Offs<T, 5> &, T, T, unsigned *, cudaStream_t, int, int, int64_t, int);
+                         const PhysT<T> &, const Offs<T, 5> &, T, T, unsigned *, cudaStream_t, int, int, int64_t, int,
+                         int64_t);
   // whether stage_k takes a first element > 0 (an element range) for arrays
   // aligned like these: (Qin, rhs, vgeo, sgeo)
   bool (*ranged)(const void *, const void *, const void *, const void *);
   bool mma;          // whether the tensor-core stage is built for this shape
-  bool mma_default;  // whether it is the shape's default stage kernel
   bool lean;         // whether the lean pipelined stage is built for this shape
-  int default_kernel;  // the stage kernel choice 0 resolves to (1 to 4)
-  int gravity_kernel;  // the same where gravity acts
+  bool march;        // whether the inviscid column march is
+  // the kernel that choice 0 resolves to (1 to 5) on a mesh of so many elements
+  // (viscous form, gravity)
+  int (*choice)(int64_t, bool, bool);
   cudaError_t (*build_nbr)(int32_t *, const int64_t *, const int64_t *, const int64_t *, int64_t,
                            unsigned *, cudaStream_t);
   // the same with neighbours allowed up to a total element count (ghosts)
@@ -55,7 +58,7 @@ struct Ops {
   cudaError_t (*cons_sums)(const T *, const T *, int64_t, int, const Offs<double, 5> &, double *, int,
                            cudaStream_t);
   // fused viscous passes over one mesh: pass 0 (gradient) or 1 (stage +
-  // update); the last arguments are the solver's kernel choice and whether the
+  // update); the last arguments are the kernel (1, 3 or 5) and whether the
   // stream's preceding launch is a pass of the same solve
   cudaError_t (*ns_pass)(int, const BDesc<T> &, T *, int64_t, const PhysT<T> &, T, T, cudaStream_t, int, int);
   // whether the viscous form of this order has stage calls, ghosts and state

@@ -82,6 +82,13 @@ bool ns_stage_form(const cb_solver *s) {
 // where the fused viscous passes raise the status: the orders without a stage
 // form do not report a non-finite state
 unsigned *visc_status(const cb_solver *s) { return ns_stage_form(s) ? s->status : s->status + 1; }
+// The kernel that the solver runs: its choice, or what the mesh defaults to.
+int kernel_of(const cb_solver *s) {
+  if (s->kernel) return s->kernel;
+  if (s->unfused) return 1;
+  const bool visc = s->phys.visc > 0, grav = s->phys.gravity != 0;
+  return s->prec == 64 ? ops<double>(s)->choice(s->nelem, visc, grav) : ops<float>(s)->choice(s->nelem, visc, grav);
+}
 // the state ping-pongs between Q and Qalt (two steps per graph)
 bool pingpong(const cb_solver *s) { return s->phys.visc <= 0 || fused_visc(s); }
 
@@ -107,10 +114,10 @@ cudaError_t enqueue_step(cb_solver *s, double dt, bool from_user, bool chained) 
     for (int st = 0; st < 5 && e == cudaSuccess; ++st) {
       I.Q[0] = a;
       I.Q[1] = b;
-      if ((e = o->ns_pass(0, I, (T *)s->gradQ, s->nelem, p, T(0), T(0), s->stream, s->kernel,
+      if ((e = o->ns_pass(0, I, (T *)s->gradQ, s->nelem, p, T(0), T(0), s->stream, kernel_of(s),
                           chained || st)) != cudaSuccess)
         break;
-      e = o->ns_pass(1, I, (T *)s->gradQ, s->nelem, p, T(RKA[(st + 1) % 5]), T(RKB[st] * dt), s->stream, s->kernel,
+      e = o->ns_pass(1, I, (T *)s->gradQ, s->nelem, p, T(RKA[(st + 1) % 5]), T(RKB[st] * dt), s->stream, kernel_of(s),
                      1);
       T *t = a;
       a = b;
@@ -137,7 +144,7 @@ cudaError_t enqueue_step(cb_solver *s, double dt, bool from_user, bool chained) 
   for (int k = 0; k < 5; ++k) q5.v[k] = T(s->qref[k]);
   for (int st = 0; st < 5 && e == cudaSuccess; ++st) {
     e = o->stage_k(a, b, (T *)s->rhs, vg, sg, s->nbr, D, s->nelem, p, q5, T(RKA[(st + 1) % 5]),
-                   T(RKB[st] * dt), s->status, s->stream, 0, s->kernel, 0, chained || st);
+                   T(RKB[st] * dt), s->status, s->stream, 0, s->kernel, 0, chained || st, s->nelem);
     T *t = a;
     a = b;
     b = t;
@@ -197,7 +204,7 @@ cudaError_t settle(cb_solver *s) {
 // The column-march passes (3-D) keep the gradient as records (grad_at), the
 // other passes as (Np, nstate, dim, elements): the form of the kernel choice.
 bool records_wanted(const cb_solver *s) {
-  return fused_visc(s) && s->dim == 3 && (s->kernel == 0 || !ns_stage_form(s));
+  return fused_visc(s) && s->dim == 3 && (kernel_of(s) == 5 || !ns_stage_form(s));
 }
 // the form the buffer is in (one that holds nothing yet is in any form)
 bool records(cb_solver *s) {
@@ -298,17 +305,17 @@ cudaError_t enqueue_pass(cb_solver *s, int st, double dt, int pass) {
     cudaError_t e = pass == 0 ? adopt_form_anew(s) : adopt_form(s);
     if (e != cudaSuccess) return e;
     if (pass == 0) {
-      e = o->ns_pass(0, I, (T *)s->gradQ, s->nelem, p, T(0), T(0), s->stream, s->kernel, 0);
+      e = o->ns_pass(0, I, (T *)s->gradQ, s->nelem, p, T(0), T(0), s->stream, kernel_of(s), 0);
       return e == cudaSuccess && records(s) ? density_gradient(s, a) : e;
     }
     if ((e = complete_gradient(s)) != cudaSuccess) return e;  // the stage may overwrite rho_src
-    return o->ns_pass(1, I, (T *)s->gradQ, s->nelem, p, T(RKA[(st + 1) % 5]), T(RKB[st] * dt), s->stream, s->kernel, 0);
+    return o->ns_pass(1, I, (T *)s->gradQ, s->nelem, p, T(RKA[(st + 1) % 5]), T(RKB[st] * dt), s->stream, kernel_of(s), 0);
   }
   if (pass == 0) return cudaSuccess;
   Offs<T, 5> q5;
   for (int k = 0; k < 5; ++k) q5.v[k] = T(s->qref[k]);
   return o->stage_k(a, b, (T *)s->rhs, (const T *)s->vgeo, (const T *)s->sgeo, s->nbr, (const T *)s->D, s->nelem,
-                    p, q5, T(RKA[(st + 1) % 5]), T(RKB[st] * dt), s->status, s->stream, 0, s->kernel, 0, 0);
+                    p, q5, T(RKA[(st + 1) % 5]), T(RKB[st] * dt), s->status, s->stream, 0, s->kernel, 0, 0, s->nelem);
 }
 
 // Copy whole elements: gather `n` elements listed in `idx` (device int64) of
@@ -467,14 +474,14 @@ int cb_solver_stage_split(cb_solver *s, int stage, double dt, int half, void **n
       e = ops<double>(s)->stage_k((const double *)a, (double *)b, (double *)s->rhs, (const double *)s->vgeo,
                                   (const double *)s->sgeo, s->nbr, (const double *)s->D, hi, PhysT<double>(ph), q5,
                                   RKA[(stage + 1) % 5], RKB[stage] * dt, s->status, s->stream, 0, s->kernel, lo,
-                                  0);
+                                  0, s->nelem);
     } else {
       Offs<float, 5> q5;
       for (int k = 0; k < 5; ++k) q5.v[k] = (float)s->qref[k];
       e = ops<float>(s)->stage_k((const float *)a, (float *)b, (float *)s->rhs, (const float *)s->vgeo,
                                  (const float *)s->sgeo, s->nbr, (const float *)s->D, hi, PhysT<float>(ph), q5,
                                  (float)RKA[(stage + 1) % 5], (float)(RKB[stage] * dt), s->status, s->stream, 0,
-                                 s->kernel, lo, 0);
+                                 s->kernel, lo, 0, s->nelem);
     }
   }
   if (e != cudaSuccess) return solver_fail(CB_ERR_CUDA, "cb_solver_stage_split: %s", cudaGetErrorString(e));
@@ -788,7 +795,7 @@ int cb_solver_set_offset(cb_solver *s, const double *qref) {
 }
 
 int cb_solver_set_kernel(cb_solver *s, int kernel) {
-  if (!s || kernel < 0 || kernel > 4) return solver_fail(CB_ERR_ARG, "cb_solver_set_kernel: bad arguments");
+  if (!s || kernel < 0 || kernel > 5) return solver_fail(CB_ERR_ARG, "cb_solver_set_kernel: bad arguments");
   if (kernel == 4) {
     const bool lean = s->prec == 64 ? ops<double>(s)->lean : ops<float>(s)->lean;
     if (!lean || s->phys.visc > 0)
@@ -800,6 +807,11 @@ int cb_solver_set_kernel(cb_solver *s, int kernel) {
       return solver_fail(CB_ERR_UNSUPPORTED,
                          "cb_solver_set_kernel: the tensor-core stage is built for the inviscid 3-D N=7 form");
   }
+  if (kernel == 5) {
+    const bool march = s->prec == 64 ? ops<double>(s)->march : ops<float>(s)->march;
+    if (s->phys.visc > 0 ? s->dim == 2 || s->unfused : !march)
+      return solver_fail(CB_ERR_UNSUPPORTED, "cb_solver_set_kernel: the grid-line stages are not built for this shape");
+  }
   if (kernel != s->kernel) drop_graph(s);
   s->kernel = kernel;
   return CB_OK;
@@ -807,10 +819,7 @@ int cb_solver_set_kernel(cb_solver *s, int kernel) {
 
 int cb_solver_get_kernel(const cb_solver *s, int *kernel) {
   if (!s || !kernel) return solver_fail(CB_ERR_ARG, "cb_solver_get_kernel: null argument");
-  const bool grav = s->phys.gravity != 0;
-  const int def = s->prec == 64 ? (grav ? ops<double>(s)->gravity_kernel : ops<double>(s)->default_kernel)
-                                : (grav ? ops<float>(s)->gravity_kernel : ops<float>(s)->default_kernel);
-  *kernel = s->kernel ? s->kernel : (s->phys.visc > 0 ? 1 : def);
+  *kernel = kernel_of(s);
   return CB_OK;
 }
 
@@ -835,13 +844,13 @@ int cb_solver_test_timeout(cb_solver *s) {
     for (int k = 0; k < 5; ++k) q5.v[k] = s->qref[k];
     e = ops<double>(s)->stage_k((const double *)a, (double *)b, (double *)s->rhs, (const double *)s->vgeo,
                                 (const double *)s->sgeo, s->nbr, (const double *)s->D, s->nelem, p64, q5, RKA[1],
-                                RKB[0], s->status, s->stream, 1, s->kernel, 0, 0);
+                                RKB[0], s->status, s->stream, 1, s->kernel, 0, 0, s->nelem);
   } else {
     Offs<float, 5> q5;
     for (int k = 0; k < 5; ++k) q5.v[k] = (float)s->qref[k];
     e = ops<float>(s)->stage_k((const float *)a, (float *)b, (float *)s->rhs, (const float *)s->vgeo,
                                (const float *)s->sgeo, s->nbr, (const float *)s->D, s->nelem, p32, q5,
-                               (float)RKA[1], (float)RKB[0], s->status, s->stream, 1, s->kernel, 0, 0);
+                               (float)RKA[1], (float)RKB[0], s->status, s->stream, 1, s->kernel, 0, 0, s->nelem);
   }
   if (e == cudaErrorNotSupported)  // returned by the launcher, not by CUDA
     return solver_fail(CB_ERR_UNSUPPORTED, "cb_solver_test_timeout: this shape does not run the pipelined stage");

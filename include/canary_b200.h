@@ -184,20 +184,22 @@ int cb_solver_sums(cb_solver *s, double *out_host);
  * non-finite state) into *out_host (page-locked memory for an asynchronous
  * copy); the value is valid once the stream has reached the copy. */
 int cb_solver_status_async(cb_solver *s, unsigned *out_host);
-/* Stage kernel: 0 = the default for the shape, 1 = the CUDA-core stages
+/* Stage kernel: 0 = the default for the mesh, 1 = the CUDA-core stages
  * (pipelined bulk-copy staging where the plan fits), 2 = the tensor-core
  * stage of the inviscid form (D contraction on the FP64 tensor pipe as 8x8x4
  * DMMA tiles, for FP32 solvers on the FP32 fluxes converted to FP64, the sum
  * rounded once; built for 3-D N=7, CB_ERR_UNSUPPORTED elsewhere), 3 = the
- * unpipelined grouped stages (the inviscid k_stage, the column march at 3-D
- * N=10 and FP64 N=8, 9; for the fused viscous form the grouped passes), 4 = the lean
+ * unpipelined grouped stages (the inviscid k_stage; for the fused viscous form
+ * the grouped passes), 4 = the lean
  * pipelined stage of the inviscid form (only the state staged in shared
- * memory, the geometry and carry read from L2; bit-identical to 1).  The
- * default is the fastest on B200 for the shape (viscous 3-D: the grid-line
- * passes, with 1 the pipelined ones up to N=7; 3-D N >= 8 has only the
- * grid-line passes).  All agree with the oracle
+ * memory, the geometry and carry read from L2; bit-identical to 1), 5 = the
+ * grid-line stages (inviscid 3-D N=10 and FP64 N=8, 9; viscous 3-D;
+ * CB_ERR_UNSUPPORTED elsewhere).  The default is the fastest on B200 for the
+ * shape and size.  Viscous 3-D N >= 8 has only the grid-line passes (face maps
+ * that are not conforming: the reference's sequence of passes), whatever the
+ * choice.  All agree with the oracle
  * to round-off; changing it re-captures the step graph at the next run.
- * cb_solver_get_kernel reports the kernel the solver runs (1 to 4). */
+ * cb_solver_get_kernel reports the kernel the solver runs (1 to 5). */
 int cb_solver_set_kernel(cb_solver *s, int kernel);
 int cb_solver_get_kernel(const cb_solver *s, int *kernel);
 /* Clear the solver's sticky status bits (stream-ordered). */
