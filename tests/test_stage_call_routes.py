@@ -1,6 +1,7 @@
 """Stage calls and runs take the same kernels, and report them.
 
-Bit for bit: a stage run in two halves against the stage in one call; a run under the
+Bit for bit: a stage run in two halves against the stage in one call; a run of a graph
+of programmatic launches against plainly launched stage calls; a run under the
 kernel that the solver reports against a run under its default."""
 import ctypes as C
 import math
@@ -56,6 +57,26 @@ def test_split_stage_equals_the_stage(dim, N, n, gravity, precision):
         check(_lib.lib().cb_solver_stage(a._h, k % 5, dt, C.byref(nxt)))
         for half in (0, 1):
             check(_lib.lib().cb_solver_stage_split(b._h, k % 5, dt, half, C.byref(nxt)))
+    assert np.array_equal(state(a), state(b))
+    a.close()
+    b.close()
+
+
+# chained launches by kernel: the small-mesh form, the grouped stage above eight
+# blocks an SM (3-D N=4 FP32, two elements a block: 14^3), the pipelined, lean,
+# tensor-core and grid-line stages, both viscous passes of each
+@pytest.mark.parametrize("dim,N,n,precision,visc", [
+    (2, 4, 10, 64, 0.0), (2, 7, 40, 64, 0.0), (2, 4, 60, 32, 0.0), (2, 7, 30, 64, 0.02), (2, 4, 20, 32, 0.02),
+    (3, 3, 9, 64, 0.0), (3, 4, 14, 32, 0.0), (3, 4, 8, 64, 0.0), (3, 5, 8, 64, 0.0), (3, 7, 8, 64, 0.0),
+    (3, 7, 8, 32, 0.0), (3, 10, 4, 64, 0.0), (3, 3, 4, 64, 0.02), (3, 3, 17, 32, 0.02), (3, 5, 4, 32, 0.02),
+    (3, 7, 10, 64, 0.02)])
+def test_run_equals_stage_calls(dim, N, n, precision, visc):
+    m, Q, dt = case(dim, N, n)
+    a, b = (solver(m, Q, precision, dict(dg.WORKLOAD_PHYS, visc=visc)) for _ in range(2))
+    a.run(4, dt)
+    nxt = C.c_void_p()
+    for k in range(20):
+        check(_lib.lib().cb_solver_stage(b._h, k % 5, dt, C.byref(nxt)))
     assert np.array_equal(state(a), state(b))
     a.close()
     b.close()
