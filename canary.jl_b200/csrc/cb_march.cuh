@@ -555,7 +555,7 @@ template <int Nq, typename T>
 __global__ void __launch_bounds__(March<Nq, T>::THREADS, March<Nq, T>::blocks_for(March<Nq, T>::REGS_GRAD))
     k_line_grad(MarchArgs<T> A, PhysT<T> p) {
   using C = March<Nq, T>;
-  constexpr int Np = C::Np, N2 = C::N2, NS = 5, NVG = 14, NSG = 5, IR = 3, MJF = 9, GC = 13, EPB = C::EPB, QR = C::QR,
+  constexpr int Np = C::Np, N2 = C::N2, NS = 5, NVG = 14, NSG = 5, IR = 3, MJF = 9, MJIF = 10, GC = 13, EPB = C::EPB, QR = C::QR,
                 QE = C::QE, VW = C::VW;
   using V = typename Vec16<T>::type;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -643,7 +643,7 @@ __global__ void __launch_bounds__(March<Nq, T>::THREADS, March<Nq, T>::blocks_fo
 #pragma unroll
       for (int s = 0; s < 4; ++s) c.Qs[s * QE + line_slab<Nq, QR, 2>(c.a, c.b, x)] *= MJ[x];
 #pragma unroll
-  for (int x = 0; x < Nq; ++x) MJ[x] = T(1) / MJ[x];
+  for (int x = 0; x < Nq; ++x) MJ[x] = c.vg[ab + N2 * x + Np * MJIF];  // from here on MJI
   cp_async_wait<2>();
   __syncthreads();  // MJ prim and the first field
   T *__restrict__ gq = A.gq + c.e * (Np * GREC);
