@@ -971,6 +971,15 @@ struct Launch {
   static bool small_mesh(int64_t nelem) {
     return EARLY_OK && (nelem + C::EPB - 1) / C::EPB <= (int64_t)EARLY_BLOCKS * num_sms();
   }
+  // Whether a chained launch of a persistent kernel of `grid` blocks is
+  // programmatic.  What overlaps is its prologue; what it costs is the even spread
+  // of the blocks: they start wherever an SM has room, so that blocks with a group
+  // more than the others meet on one SM.  Worth it where every block has one group or
+  // the prologue zeroes padded flux rows (2-D, us a step plain / programmatic: FP64
+  // N=4 60^2 42.1 / 39.0, FP32 N=5 72^2 42.1 / 39.2; unpadded with 1.35 groups a block,
+  // N=7 40^2 34.9 / 38.0; 3-D N=7 FP32 24^3 1118 / 1186, N=3 FP64 40^3 1555 / 1640).
+  static constexpr bool PADDED = Pipe2<DIM, Nq, T>::MV > Nq;
+  static int chain_pays(int chained, int64_t groups, int64_t grid) { return chained && (PADDED || groups <= grid); }
   // The stage kernel that choice 0 resolves to on a mesh of nelem elements.
   static int choice(int64_t nelem, bool gravity) {
     if (MARCH) return 5;
@@ -1036,7 +1045,7 @@ struct Launch {
       if (kernel == 5) {
         MarchArgs<T> a{Qin, Qout, rhs, vgeo, sgeo, nbr, D, nullptr, ebeg, nelem, {}, rka, rkbdt, status};
         for (int s = 0; s < NS; ++s) a.qref.v[s] = qref.v[s];
-        return march_stage<T>(Nq, false, a, p, st, chained);
+        return march_stage<T>(Nq, false, a, p, st);
       }
     }
     if (kernel == 5 || (kernel == 2 && !(MMA_OK && aligned2))) return cudaErrorNotSupported;
@@ -1050,7 +1059,10 @@ struct Launch {
         const size_t sm = smem_stage();
         const cudaError_t err = prep(k_stage<DIM, Nq, T, true>, sm);
         if (err != cudaSuccess) return err;
-        return launch_stage_kernel(k_stage<DIM, Nq, T, true>, (unsigned)groups, C::THREADS, sm, st, chained, Qin, Qout,
+        // (2-D: plain above 2.5 blocks per SM, where they no longer spread evenly, FP32
+        // N=7 40^2 20.2 us a step against 23.6, N=4 60^2, 2.4 blocks per SM, 23.2 against 20.5)
+        const int chain = chained && (DIM == 3 || 2 * groups <= 5 * num_sms());
+        return launch_stage_kernel(k_stage<DIM, Nq, T, true>, (unsigned)groups, C::THREADS, sm, st, chain, Qin, Qout,
                                    rhs, vgeo, sgeo, nbr, D, nelem, p, qref, rka, rkbdt, status, ebeg);
       }
     }
@@ -1065,7 +1077,8 @@ struct Launch {
         int64_t g = (int64_t)num_sms() * bps;
         if (g > groups) g = groups;
         const S src{Qin, Qout, rhs, vgeo, sgeo, nbr, D, nelem, qref, rkbdt, status, probe, ebeg};
-        return launch_stage_kernel(k_stage_mma<S, PM::MINB>, (unsigned)g, PM::THREADS, PM::smem(), st, chained, src, p, rka);
+        return launch_stage_kernel(k_stage_mma<S, PM::MINB>, (unsigned)g, PM::THREADS, PM::smem(), st,
+                                   chain_pays(chained, groups, g), src, p, rka);
       }
     }
     if constexpr (LEAN_OK) {
@@ -1079,7 +1092,8 @@ struct Launch {
         int64_t g = (int64_t)num_sms() * bps;
         if (g > groups) g = groups;
         const S src{Qin, Qout, rhs, vgeo, sgeo, nbr, D, nelem, qref, rkbdt, status, probe, ebeg};
-        return launch_stage_kernel(k_stage_lean<DIM, Nq, T, S>, (unsigned)g, C::THREADS, PL::smem(), st, chained, src, p, rka);
+        return launch_stage_kernel(k_stage_lean<DIM, Nq, T, S>, (unsigned)g, C::THREADS, PL::smem(), st,
+                                   chain_pays(chained, groups, g), src, p, rka);
       }
     }
     if (Pipe2<DIM, Nq, T>::OK && aligned2 && kernel != 3) {
@@ -1093,7 +1107,8 @@ struct Launch {
       int64_t g = (int64_t)num_sms() * bps;
       if (g > groups) g = groups;
       const S src{Qin, Qout, rhs, vgeo, sgeo, nbr, D, nelem, qref, rkbdt, status, probe, ebeg};
-      return launch_stage_kernel(k_stage_pipe2<DIM, Nq, T, S>, (unsigned)g, C::THREADS, sm, st, chained, src, p, rka);
+      return launch_stage_kernel(k_stage_pipe2<DIM, Nq, T, S>, (unsigned)g, C::THREADS, sm, st,
+                                 chain_pays(chained, groups, g), src, p, rka);
     } else if (probe || (ebeg && kernel != 3)) {
       return cudaErrorNotSupported;
     } else if (pipe_ok && aligned && kernel != 3) {

@@ -203,7 +203,6 @@ __global__ void __launch_bounds__(March<Nq, T>::THREADS,
   T *DT = reinterpret_cast<T *>(smem_raw + C::OFF_DT), *DZ = reinterpret_cast<T *>(smem_raw + C::OFF_DZ);
   T *PL = reinterpret_cast<T *>(smem_raw + C::OFF_P);
   T *FF = reinterpret_cast<T *>(smem_raw + C::OFF_FF);
-  grid_wait(a.Qin, a.Qout, a.rhs, a.gq);
   const int tid = threadIdx.x, el = tid / N2, ij = tid % N2, i = ij % Nq, j = ij / Nq;
   const int64_t e0 = a.ebeg + (int64_t)blockIdx.x * EPB, e = e0 + el;
   const bool act = el < EPB && e < a.eend;
@@ -560,7 +559,6 @@ __global__ void __launch_bounds__(March<Nq, T>::THREADS, March<Nq, T>::blocks_fo
   using V = typename Vec16<T>::type;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T *DS = reinterpret_cast<T *>(smem_raw), *S = reinterpret_cast<T *>(smem_raw + C::OFF_S);
-  grid_wait(A.Qin, A.gq);
   const int tid = threadIdx.x, el = tid / N2, ab = tid % N2;
   const int64_t e0 = A.ebeg + (int64_t)blockIdx.x * EPB;
   LineCtx<Nq, T> c;
@@ -742,19 +740,22 @@ struct MarchLaunch {
     return cudaGetLastError();
   }
   template <typename K>
-  static cudaError_t launch(K kernel, size_t smem, const MarchArgs<T> &a, const PhysT<T> &p, cudaStream_t st,
-                            int chained) {
+  static cudaError_t launch(K kernel, size_t smem, const MarchArgs<T> &a, const PhysT<T> &p, cudaStream_t st) {
     const int64_t g = (a.eend - a.ebeg + M::EPB - 1) / M::EPB;
     if (g <= 0) return cudaSuccess;
     if (smem > 48 * 1024) {
       const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return e;
     }
-    return launch_stage_kernel(kernel, (unsigned)g, M::THREADS, smem, st, chained, a, p);
+    // (plain: a programmatic launch of either kernel starts its blocks unevenly and gains
+    // nothing, us a viscous step plain / programmatic: N=7 FP32 8^3 157 / 231, 20^3 2020 / 2330,
+    // N=4 FP32 10^3 121 / 173, N=7 FP64 20^3 4080 / 4540)
+    kernel<<<(unsigned)g, M::THREADS, smem, st>>>(a, p);
+    return cudaGetLastError();
   }
-  static cudaError_t stage(bool visc, const MarchArgs<T> &a, const PhysT<T> &p, cudaStream_t st, int chained) {
-    return visc ? launch(k_march_stage<Nq, T, true>, M::smem_stage(), a, p, st, chained)
-                : launch(k_march_stage<Nq, T, false>, M::smem_stage(), a, p, st, chained);
+  static cudaError_t stage(bool visc, const MarchArgs<T> &a, const PhysT<T> &p, cudaStream_t st) {
+    return visc ? launch(k_march_stage<Nq, T, true>, M::smem_stage(), a, p, st)
+                : launch(k_march_stage<Nq, T, false>, M::smem_stage(), a, p, st);
   }
   static cudaError_t volume(T *rhs, const T *Q, const T *vgeo, const T *D, int64_t nelem, const PhysT<T> &p,
                             cudaStream_t st) {
@@ -768,8 +769,8 @@ struct MarchLaunch {
     k_march_volume<Nq, T><<<(unsigned)g, M::THREADS, M::smem_volume(), st>>>(rhs, Q, vgeo, D, nelem, p);
     return cudaGetLastError();
   }
-  static cudaError_t grad(const MarchArgs<T> &a, const PhysT<T> &p, cudaStream_t st, int chained) {
-    return launch(k_line_grad<Nq, T>, M::smem_grad(), a, p, st, chained);
+  static cudaError_t grad(const MarchArgs<T> &a, const PhysT<T> &p, cudaStream_t st) {
+    return launch(k_line_grad<Nq, T>, M::smem_grad(), a, p, st);
   }
 };
 
@@ -779,14 +780,13 @@ struct MarchLaunch {
 #define CB_MARCH_DEFINE(T_)                                                                                         \
   namespace cb {                                                                                                    \
   template <>                                                                                                       \
-  cudaError_t march_stage<T_>(int Nq, bool visc, const MarchArgs<T_> &a, const PhysT<T_> &p, cudaStream_t st,       \
-                              int chained) {                                                                        \
-    static cudaError_t (*const f[])(bool, const MarchArgs<T_> &, const PhysT<T_> &, cudaStream_t, int) = {          \
+  cudaError_t march_stage<T_>(int Nq, bool visc, const MarchArgs<T_> &a, const PhysT<T_> &p, cudaStream_t st) {     \
+    static cudaError_t (*const f[])(bool, const MarchArgs<T_> &, const PhysT<T_> &, cudaStream_t) = {               \
         &MarchLaunch<2, T_>::stage, &MarchLaunch<3, T_>::stage, &MarchLaunch<4, T_>::stage,                         \
         &MarchLaunch<5, T_>::stage, &MarchLaunch<6, T_>::stage, &MarchLaunch<7, T_>::stage,                         \
         &MarchLaunch<8, T_>::stage, &MarchLaunch<9, T_>::stage, &MarchLaunch<10, T_>::stage,                        \
         &MarchLaunch<11, T_>::stage};                                                                               \
-    return Nq < 2 || Nq > 11 ? cudaErrorInvalidValue : f[Nq - 2](visc, a, p, st, chained);                          \
+    return Nq < 2 || Nq > 11 ? cudaErrorInvalidValue : f[Nq - 2](visc, a, p, st);                                   \
   }                                                                                                                 \
   template <>                                                                                                       \
   cudaError_t march_volume<T_>(int Nq, T_ *rhs, const T_ *Q, const T_ *vgeo, const T_ *D, int64_t nelem,            \
@@ -800,12 +800,12 @@ struct MarchLaunch {
     return Nq < 2 || Nq > 11 ? cudaErrorInvalidValue : f[Nq - 2](rhs, Q, vgeo, D, nelem, p, st);                    \
   }                                                                                                                 \
   template <>                                                                                                       \
-  cudaError_t march_grad<T_>(int Nq, const MarchArgs<T_> &a, const PhysT<T_> &p, cudaStream_t st, int chained) {    \
-    static cudaError_t (*const f[])(const MarchArgs<T_> &, const PhysT<T_> &, cudaStream_t, int) = {                \
+  cudaError_t march_grad<T_>(int Nq, const MarchArgs<T_> &a, const PhysT<T_> &p, cudaStream_t st) {                 \
+    static cudaError_t (*const f[])(const MarchArgs<T_> &, const PhysT<T_> &, cudaStream_t) = {                     \
         &MarchLaunch<2, T_>::grad, &MarchLaunch<3, T_>::grad, &MarchLaunch<4, T_>::grad, &MarchLaunch<5, T_>::grad, \
         &MarchLaunch<6, T_>::grad, &MarchLaunch<7, T_>::grad, &MarchLaunch<8, T_>::grad, &MarchLaunch<9, T_>::grad, \
         &MarchLaunch<10, T_>::grad, &MarchLaunch<11, T_>::grad};                                                    \
-    return Nq < 2 || Nq > 11 ? cudaErrorInvalidValue : f[Nq - 2](a, p, st, chained);                                \
+    return Nq < 2 || Nq > 11 ? cudaErrorInvalidValue : f[Nq - 2](a, p, st);                                         \
   }                                                                                                                 \
   template <>                                                                                                       \
   cudaError_t density_gradient<T_>(int Nq, const T_ *Q, T_ *out, const T_ *vgeo, const T_ *sgeo,                    \

@@ -26,15 +26,15 @@ struct MarchArgs {
 };
 
 // Fused stage of order Nq - 1 (visc: the second viscous pass) and the
-// gradient pass (chained: see launch_stage_kernel).
+// gradient pass.
 template <typename T>
-cudaError_t march_stage(int Nq, bool visc, const MarchArgs<T> &a, const PhysT<T> &p, cudaStream_t st, int chained);
+cudaError_t march_stage(int Nq, bool visc, const MarchArgs<T> &a, const PhysT<T> &p, cudaStream_t st);
 // rhs += volume integral (volumerhs!).
 template <typename T>
 cudaError_t march_volume(int Nq, T *rhs, const T *Q, const T *vgeo, const T *D, int64_t nelem, const PhysT<T> &p,
                          cudaStream_t st);
 template <typename T>
-cudaError_t march_grad(int Nq, const MarchArgs<T> &a, const PhysT<T> &p, cudaStream_t st, int chained);
+cudaError_t march_grad(int Nq, const MarchArgs<T> &a, const PhysT<T> &p, cudaStream_t st);
 // Density gradient (Np, 3, nelem) of the state Q, which the records leave out (it
 // does not enter the viscous flux): for callers who take the whole gradient.
 template <typename T>
