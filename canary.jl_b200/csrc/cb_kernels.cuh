@@ -935,7 +935,10 @@ struct Launch {
   // N=10 FP64 4.28 -> 3.35, FP32 1.92 -> 1.61; N=9 FP64 2.96 -> 2.72; N=8 FP64
   // 16^3 1.58 -> 1.43, under gravity 1.64 -> 1.45).  Below,
   // the other stages are the faster ones (N=9 FP32 grouped 1.36, march 1.51;
-  // N=4 FP32 1.21, 1.24; N=7 FP64 tensor-core 1.75, march 2.34).
+  // N=4 FP32 1.21, 1.24; N=7 FP64 tensor-core 1.75, march 2.34).  Meshes of up to an
+  // element per SM keep the grouped stage, whose block spreads an element over 512
+  // threads (5^3, us a step, grouped / march: FP64 N=8 52 / 83, N=9 65 / 84, N=10 100 /
+  // 116, FP32 N=10 64 / 75; 6^3: 99 / 106, 125 / 118, 196 / 174, 106 / 97).
   static constexpr bool MARCH = DIM == 3 && (Nq >= 11 || (Nq >= 9 && sizeof(T) == 8));
   // Default stage kernel per shape, from B200 timings of one mesh (ms per
   // step, warped 3-D cubes of 7-17 M nodes; pipelined CUDA-core / grouped /
@@ -982,7 +985,7 @@ struct Launch {
   static int chain_pays(int chained, int64_t groups, int64_t grid) { return chained && (PADDED || groups <= grid); }
   // The stage kernel that choice 0 resolves to on a mesh of nelem elements.
   static int choice(int64_t nelem, bool gravity) {
-    if (MARCH) return 5;
+    if (MARCH) return nelem <= num_sms() ? 3 : 5;
     if (DIM == 2 && small_mesh(nelem)) return 3;
     return gravity ? GRAVITY_KERNEL : DEFAULT_KERNEL;
   }
