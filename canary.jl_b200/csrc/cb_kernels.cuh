@@ -960,7 +960,12 @@ struct Launch {
   // The same under gravity, whose heights are a dependent load in every phase:
   // where more warps are in flight than in the default (B200, ms per step: FP64
   // N=6 19^3 pipelined 1.12, lean 1.08, without gravity 1.00 and 1.04; N=4 28^3
-  // lean 1.39, grouped 1.33, without gravity 1.30 and 1.32).
+  // lean 1.39, grouped 1.33, without gravity 1.30 and 1.32; N=4 is so at every size, 5^3
+  // 31 us and 29).  N=6 in large meshes only: up to two dozen elements per SM the blocks of
+  // the pipelined stage, one per SM and each the whole SM's, are the faster ones (us a
+  // step, pipelined / lean: 5^3 32 / 39, 9^3 117 / 145, 12^3 301 / 302, 15^3 565 / 566,
+  // 16^3 682 / 664, 24^3 2241 / 2145).
+  static constexpr int GRAVITY_LEAN_GROUPS = 24;
   static constexpr int GRAVITY_KERNEL = DIM == 3 && sizeof(T) == 8 && Nq == 7   ? 4
                                         : DIM == 3 && sizeof(T) == 8 && Nq == 5 ? 3
                                                                                 : DEFAULT_KERNEL;
@@ -987,6 +992,7 @@ struct Launch {
   static int choice(int64_t nelem, bool gravity) {
     if (MARCH) return nelem <= num_sms() ? 3 : 5;
     if (DIM == 2 && small_mesh(nelem)) return 3;
+    if (GRAVITY_KERNEL == 4 && DEFAULT_KERNEL == 1 && nelem <= GRAVITY_LEAN_GROUPS * num_sms()) return 1;
     return gravity ? GRAVITY_KERNEL : DEFAULT_KERNEL;
   }
   // Resident blocks per SM of a kernel at `smem` bytes, from the occupancy

@@ -60,3 +60,17 @@ def test_inviscid_high_orders(N, precision, sides):
         s.run(2, dt)
         assert max(relerr_fields(s.state(), oracle_run(m, Q, dt, 2, phys=phys))) < (1e-12 if precision == 64 else 1e-5), n
         s.close()
+
+
+@pytest.mark.parametrize("n,gravity", [(5, 0.3), (15, 0.3), (16, 0.3), (5, 0.0), (16, 0.0)])
+def test_gravity_at_order_six(n, gravity):
+    m = dg.build_mesh(3, 6, (np.linspace(0, 1, n + 1),) * 3, (True, True, False))
+    Q = np.zeros((m.Np, 5, m.nelem), order="F")
+    Q[:, 3], Q[:, 4] = 1.0, 2.5
+    phys = dict(dg.WORKLOAD_PHYS, gravity=gravity)
+    s = dg.LSRK.for_state(dg.DeviceMesh.upload(m), Q, 64, phys=dg.make_phys(**phys))
+    assert s.kernel == (4 if gravity and m.nelem > 24 * sms() else 1)
+    if n == 5:
+        s.run(2, 1e-4)
+        assert max(relerr_fields(s.state() + 1.0, oracle_run(m, Q, 1e-4, 2, phys=phys) + 1.0)) < 1e-12
+    s.close()
