@@ -904,8 +904,16 @@ struct Launch {
                                const PhysT<T> &p, cudaStream_t st) {
     // 3-D N >= 3 (FP64: 4): the march (B200, 2.3 M nodes, us: FP64 N=4 98.9 ->
     // 90.0, N=8 190.8 -> 166.2, N=10 188.6 -> 149.9, FP32 N=7 72.4 -> 57.9; below,
-    // the grouped kernel is the faster one: FP64 N=3 72.5, march 74.1)
-    if constexpr (DIM == 3 && Nq >= (sizeof(T) == 4 ? 4 : 5)) return march_volume<T>(Nq, rhs, Q, vgeo, D, nelem, p, st);
+    // the grouped kernel is the faster one: FP64 N=3 72.5, march 74.1).  The grouped
+    // kernel spreads a node's work over more threads and is the faster one up to so
+    // many of its blocks per SM (us a call, grouped / march: FP64 N=4 5^3 3.2 / 6.4, 12^3
+    // 10.2 / 11.3, 20^3 46.6 / 44.3; N=5 7^3 5.2 / 6.1, 10^3 9.8 / 9.1; N=7 5^3 5.3 / 6.2, 8^3
+    // 15.4 / 11.2; N=10 5^3 13.7 / 14.4; FP32 N=3 10^3 2.8 / 3.0, 15^3 4.8 / 4.5; N=6 6^3 4.5 /
+    // 6.6, 9^3 8.3 / 8.3; N=9 4^3 6.0 / 6.7, 6^3 9.8 / 8.5).
+    if constexpr (DIM == 3 && Nq >= (sizeof(T) == 4 ? 4 : 5)) {
+      constexpr int GROUPED_BLOCKS = Nq >= 9 ? 1 : Nq == 5 ? 8 : 3;
+      if (grid(nelem) > GROUPED_BLOCKS * num_sms()) return march_volume<T>(Nq, rhs, Q, vgeo, D, nelem, p, st);
+    }
     size_t sm = smem_volume();
     cudaError_t err = prep(k_volumerhs<DIM, Nq, T>, sm);
     if (err != cudaSuccess) return err;
