@@ -41,9 +41,9 @@ struct cb_solver {
   // form the gradient buffer is in: 0 not written yet, 1 (Np, nstate, dim,
   // elements), 2 records (grad_at)
   int grad_form = 0;
-  // records: the state (input of the last stage of a run) whose density
-  // gradient the buffer still lacks; no pass reads it, so it is formed when
-  // the gradient is packed
+  // records: the state (Q or the twin, the input of the last gradient pass)
+  // whose density gradient the buffer still lacks; no pass reads it, so it is
+  // formed when the gradient is packed or that state is about to change
   const void *rho_src = nullptr;
   cb_phys phys{};
   cudaStream_t stream = nullptr;
@@ -194,13 +194,6 @@ size_t state_bytes(const cb_solver *s) {
   return (s->prec == 64 ? 8 : 4) * (size_t)Np * (s->dim == 2 ? 4 : 5) * s->nelem;
 }
 
-// bring the state back into the caller's Q after an odd number of stages
-cudaError_t settle(cb_solver *s) {
-  if (!s->cur) return cudaSuccess;
-  s->cur = 0;
-  return cudaMemcpyAsync(s->Q, s->Qalt, state_bytes(s), cudaMemcpyDeviceToDevice, s->stream);
-}
-
 // The column-march passes (3-D) keep the gradient as records (grad_at), the
 // other passes as (Np, nstate, dim, elements): the form of the kernel choice.
 bool records_wanted(const cb_solver *s) {
@@ -228,8 +221,19 @@ cudaError_t density_gradient(cb_solver *s, const void *src) {
 cudaError_t density_gradient(cb_solver *s, const void *src) {
   return s->prec == 64 ? density_gradient<double>(s, src) : density_gradient<float>(s, src);
 }
-// the whole gradient, as far as a run left it
-cudaError_t complete_gradient(cb_solver *s) { return s->rho_src ? density_gradient(s, s->rho_src) : cudaSuccess; }
+// the whole gradient; with `about_to_change`, only if it lacks that state's
+cudaError_t complete_gradient(cb_solver *s, const void *about_to_change = nullptr) {
+  if (!s->rho_src || (about_to_change && about_to_change != s->rho_src)) return cudaSuccess;
+  return density_gradient(s, s->rho_src);
+}
+// bring the state back into the caller's Q after an odd number of stages
+cudaError_t settle(cb_solver *s) {
+  if (!s->cur) return cudaSuccess;
+  const cudaError_t e = complete_gradient(s, s->Q);
+  if (e != cudaSuccess) return e;
+  s->cur = 0;
+  return cudaMemcpyAsync(s->Q, s->Qalt, state_bytes(s), cudaMemcpyDeviceToDevice, s->stream);
+}
 
 // Value of gradient component d of field s5 at a node in the records' form of
 // a buffer of `nall` elements: [nall][Np][GREC] for u, v, w and T, then
@@ -305,10 +309,10 @@ cudaError_t enqueue_pass(cb_solver *s, int st, double dt, int pass) {
     cudaError_t e = pass == 0 ? adopt_form_anew(s) : adopt_form(s);
     if (e != cudaSuccess) return e;
     if (pass == 0) {
-      e = o->ns_pass(0, I, (T *)s->gradQ, s->nelem, p, T(0), T(0), s->stream, kernel_of(s), 0);
-      return e == cudaSuccess && records(s) ? density_gradient(s, a) : e;
+      s->rho_src = records(s) ? a : nullptr;
+      return o->ns_pass(0, I, (T *)s->gradQ, s->nelem, p, T(0), T(0), s->stream, kernel_of(s), 0);
     }
-    if ((e = complete_gradient(s)) != cudaSuccess) return e;  // the stage may overwrite rho_src
+    if ((e = complete_gradient(s, b)) != cudaSuccess) return e;
     return o->ns_pass(1, I, (T *)s->gradQ, s->nelem, p, T(RKA[(st + 1) % 5]), T(RKB[st] * dt), s->stream, kernel_of(s), 0);
   }
   if (pass == 0) return cudaSuccess;
@@ -352,23 +356,45 @@ cudaError_t grad_elems(cb_solver *s, bool pack, const int64_t *idx, int64_t firs
 
 // After an odd number of steps of a run whose gradient is kept as records: the
 // state goes back from the twin into Q, and the density of Q, which the last
-// stage read, into the twin (see rho_src).
+// stage read, into the twin (see rho_src).  One pass over memory: eight loads in
+// flight and one division per thread (with a division per value 10 us more on 35 MB).
+constexpr int COPY_BACK = 8;
 template <typename T, typename I>
-__global__ void k_copy_back(T *__restrict__ Q, T *__restrict__ twin, I Np, I total) {
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    const T v = twin[t];
-    if ((I)t / Np % 5 == 3) twin[t] = Q[t];
-    Q[t] = v;
+__global__ void __launch_bounds__(256) k_copy_back(T *__restrict__ Q, T *__restrict__ twin, uint32_t Np, uint32_t inv,
+                                                   int64_t total) {
+  const int64_t t0 = blockIdx.x * (int64_t)(256 * COPY_BACK);
+  const uint32_t r0 = (uint32_t)((I)t0 % (5 * Np)), w = 5 * Np;
+  // (inv = 2^32 / w rounded up: exact quotients for r < w + 2048 <= 8703)
+  auto density = [&](uint32_t d) {
+    const uint32_t r = r0 + d, m = r - __umulhi(r, inv) * w;
+    return m >= 3 * Np && m < 4 * Np;
+  };
+  T v[COPY_BACK], rho[COPY_BACK];
+#pragma unroll
+  for (int k = 0; k < COPY_BACK; ++k) {
+    const uint32_t d = threadIdx.x + 256 * k;
+    if (t0 + d < total) {
+      v[k] = twin[t0 + d];
+      if (density(d)) rho[k] = Q[t0 + d];
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < COPY_BACK; ++k) {
+    const uint32_t d = threadIdx.x + 256 * k;
+    if (t0 + d < total) {
+      if (density(d)) twin[t0 + d] = rho[k];
+      Q[t0 + d] = v[k];
+    }
   }
 }
 template <typename T>
 cudaError_t copy_back(cb_solver *s) {
   const int64_t Np = nodes(s), total = Np * 5 * s->nelem;
-  const unsigned grid = blocks_for(total);
-  if (total <= 0xffffffffll)
-    k_copy_back<T, uint32_t><<<grid, 256, 0, s->stream>>>((T *)s->Q, (T *)s->Qalt, (uint32_t)Np, (uint32_t)total);
-  else
-    k_copy_back<T, int64_t><<<grid, 256, 0, s->stream>>>((T *)s->Q, (T *)s->Qalt, Np, total);
+  const unsigned grid = (unsigned)((total + 256 * COPY_BACK - 1) / (256 * COPY_BACK));
+  const uint32_t inv = (uint32_t)(((uint64_t)1 << 32) / (uint64_t)(5 * Np)) + 1;
+  T *Q = (T *)s->Q, *twin = (T *)s->Qalt;
+  if (total <= 0xffffffffll) k_copy_back<T, uint32_t><<<grid, 256, 0, s->stream>>>(Q, twin, (uint32_t)Np, inv, total);
+  else k_copy_back<T, int64_t><<<grid, 256, 0, s->stream>>>(Q, twin, (uint32_t)Np, inv, total);
   return cudaGetLastError();
 }
 
@@ -408,7 +434,7 @@ cudaError_t launch_faces(cb_solver *s, bool pack, int what, const int64_t *codes
   const int W = (s->dim == 2 ? 4 : 5) * (what ? s->dim : 1);
   T *arr = (T *)(what ? s->gradQ : (s->cur ? s->Qalt : s->Q));
   const bool rec = what && records(s);
-  const cudaError_t e = what ? complete_gradient(s) : cudaSuccess;
+  const cudaError_t e = what ? complete_gradient(s) : pack ? cudaSuccess : complete_gradient(s, arr);
   if (e != cudaSuccess) return e;
   const int64_t total = n * W * Nfp;
   const int grid = (int)std::min<int64_t>((total + 255) / 256, 148 * 16);
@@ -573,7 +599,8 @@ int cb_solver_unpack(cb_solver *s, int what, const void *buf, int64_t first, int
   } else {
     const size_t ew = state_bytes(s) / (size_t)s->nelem * (what ? s->dim : 1);
     char *dst = (char *)(what ? s->gradQ : (s->cur ? s->Qalt : s->Q)) + ew * (size_t)(s->nelem + first);
-    e = cudaMemcpyAsync(dst, buf, ew * (size_t)n, cudaMemcpyDeviceToDevice, s->stream);
+    if ((e = what ? cudaSuccess : complete_gradient(s, s->cur ? s->Qalt : s->Q)) == cudaSuccess)
+      e = cudaMemcpyAsync(dst, buf, ew * (size_t)n, cudaMemcpyDeviceToDevice, s->stream);
   }
   return e == cudaSuccess ? CB_OK : solver_fail(CB_ERR_CUDA, "cb_solver_unpack: %s", cudaGetErrorString(e));
 }
@@ -705,10 +732,10 @@ int cb_lsrk_run(cb_solver *s, int64_t nsteps, double dt) {
   if (!s) return solver_fail(CB_ERR_ARG, "null solver");
   if (nsteps < 0) return solver_fail(CB_ERR_ARG, "nsteps must be >= 0");
   if (nsteps == 0) return CB_OK;
-  cudaError_t e0 = settle(s);  // a state left in the twin by the stage API
+  cudaError_t e0 = s->phys.visc > 0 ? adopt_form_anew(s) : cudaSuccess;
+  if (e0 != cudaSuccess) return solver_fail(CB_ERR_CUDA, "gradient form: %s", cudaGetErrorString(e0));
+  e0 = settle(s);  // a state left in the twin by the stage API
   if (e0 != cudaSuccess) return solver_fail(CB_ERR_CUDA, "state copy: %s", cudaGetErrorString(e0));
-  if (s->phys.visc > 0 && (e0 = adopt_form_anew(s)) != cudaSuccess)
-    return solver_fail(CB_ERR_CUDA, "gradient form: %s", cudaGetErrorString(e0));
   const bool rec = records_wanted(s);
   const int64_t per_graph = pingpong(s) ? 2 : 1;
   const int64_t reps = nsteps / per_graph, rem = nsteps % per_graph;
@@ -726,17 +753,14 @@ int cb_lsrk_run(cb_solver *s, int64_t nsteps, double dt) {
     if ((e = enqueue(s, dt, true, false)) != cudaSuccess)
       return solver_fail(CB_ERR_CUDA, "step launch: %s", cudaGetErrorString(e));
   }
-  // records: the density gradient is left to whoever packs it, where the last
-  // stage's input stays in the twin until then
-  const void *last = rem ? s->Q : s->Qalt;
-  if (rec && s->nghost && (e = density_gradient(s, last)) != cudaSuccess)
+  // records: the density gradient is left to whoever packs it; the last stage's
+  // input (its density, where the state goes back from the twin into Q) stays in
+  // the twin until then
+  if (rec && s->nghost && (e = density_gradient(s, rem ? s->Q : s->Qalt)) != cudaSuccess)
     return solver_fail(CB_ERR_CUDA, "density gradient: %s", cudaGetErrorString(e));
   if (rec && !s->nghost) s->rho_src = s->Qalt;
-  if (rem && rec && !s->nghost) {
-    e = s->prec == 64 ? copy_back<double>(s) : copy_back<float>(s);
-  } else if (rem) {
-    e = cudaMemcpyAsync(s->Q, s->Qalt, state_bytes(s), cudaMemcpyDeviceToDevice, s->stream);
-  }
+  if (rem && s->rho_src) e = s->prec == 64 ? copy_back<double>(s) : copy_back<float>(s);
+  else if (rem) e = cudaMemcpyAsync(s->Q, s->Qalt, state_bytes(s), cudaMemcpyDeviceToDevice, s->stream);
   if (rem && e != cudaSuccess) return solver_fail(CB_ERR_CUDA, "state copy: %s", cudaGetErrorString(e));
   return CB_OK;
 }

@@ -89,7 +89,7 @@ def solver(m, Q, precision, phys, kernel=0, offset=None):
 
 
 @pytest.mark.parametrize("precision", [64, 32])
-@pytest.mark.parametrize("kernel", [0, 1, 3])
+@pytest.mark.parametrize("kernel", [5, 1, 3])
 @pytest.mark.parametrize("N,n,gravity", [(1, (3, 4, 3), 0.0), (2, (3, 3, 3), 0.0), (4, (3, 2, 3), 0.3),
                                          (7, (2, 2, 3), 0.0)])
 def test_packed_gradient_of_a_pass(N, n, gravity, kernel, precision):
@@ -123,7 +123,7 @@ def test_packed_gradient_of_a_pass(N, n, gravity, kernel, precision):
     s.close()
 
 
-@pytest.mark.parametrize("N,kernel", [(3, 0), (3, 1), (6, 0), (8, 0), (10, 0)])
+@pytest.mark.parametrize("N,kernel", [(3, 5), (3, 1), (6, 5), (8, 0), (10, 0)])
 @pytest.mark.parametrize("steps", [1, 2, 3])
 def test_packed_gradient_after_a_run(N, kernel, steps):
     """The buffer holds the gradient of the last stage, as a pass leaves it;
@@ -142,15 +142,38 @@ def test_packed_gradient_after_a_run(N, kernel, steps):
         if between == "offset" and N <= 7:
             s.set_offset([0.0, 0.0, 0.0, 0.5, 0.0])
         if between == "kernel":
-            s.set_kernel({0: 3, 1: 0}[kernel])
+            s.set_kernel({0: 3, 5: 3, 1: 5}[kernel])
         if between == "pass":
             stage_pass(s, 0, dt, 1)  # (on the gradient at hand: its values stay)
         assert gradient_error(packed(s, m, idx, torch.float64), ref[..., idx]) < 1e-10, between
         s.close()
 
 
+@pytest.mark.parametrize("between", ["none", "settle", "offset", "pass"])
+@pytest.mark.parametrize("stages", [1, 2, 3])
+@pytest.mark.parametrize("N,kernel", [(3, 5), (3, 1), (6, 5)])
+def test_packed_gradient_after_stage_calls(N, kernel, stages, between):
+    """The gradient of the last stage call, also once its input has been overwritten."""
+    import torch
+    m, Q, dt, phys = box(N, (2, 3, 2))
+    _, ref = plain_run(m, Q, dt, 0, phys, stages=stages)
+    s = solver(m, Q, 64, phys, kernel)
+    nxt = C.c_void_p()
+    for st in range(stages):
+        check(_lib.lib().cb_solver_stage(s._h, st, dt, C.byref(nxt)))
+    if between == "settle":
+        check(_lib.lib().cb_solver_settle(s._h))
+    if between == "offset":
+        s.set_offset([0.0, 0.0, 0.0, 0.5, 0.0])
+    if between == "pass":
+        stage_pass(s, stages, dt, 1)
+    idx = np.arange(m.nelem)
+    assert gradient_error(packed(s, m, idx, torch.float64), ref) < 1e-10
+    s.close()
+
+
 @pytest.mark.parametrize("precision,tol", [(64, 1e-12), (32, 1e-5)])
-@pytest.mark.parametrize("first,second", [(0, 1), (1, 0), (0, 3), (3, 0)])
+@pytest.mark.parametrize("first,second", [(5, 1), (1, 5), (5, 3), (3, 5)])
 @pytest.mark.parametrize("N", [2, 5])
 def test_kernel_choice_between_two_passes(N, first, second, precision, tol):
     m, Q, dt, phys = box(N, (3, 3, 2))
@@ -177,7 +200,7 @@ def test_parts_with_different_kernel_choices(precision, tol, faces):
     want, _ = plain_run(m, Q, dt, 2, phys)
     stream = torch.cuda.Stream()
     parts = [P.GhostedLSRK(m, P.plan(m, r, 3), Q, precision, dg.make_phys(**phys), stream=stream) for r in range(3)]
-    for part, kernel in zip(parts, (0, 1, 3)):
+    for part, kernel in zip(parts, (5, 1, 3)):
         check(_lib.lib().cb_solver_set_kernel(part._h, kernel))
     P.run_parts(parts, 2, dt, faces=faces)
     got = np.concatenate([p.state() for p in parts], axis=2)
@@ -186,7 +209,7 @@ def test_parts_with_different_kernel_choices(precision, tol, faces):
     assert max(relerr_fields(got, want)) < tol
 
 
-@pytest.mark.parametrize("before,after", [(0, 1), (1, 0)])
+@pytest.mark.parametrize("before,after", [(5, 1), (1, 5)])
 def test_ghost_gradients_outlive_a_kernel_choice(before, after):
     """Ghost gradients stored under one choice are read by a stage of another."""
     import torch

@@ -69,7 +69,7 @@ def test_split_stage_equals_the_stage(dim, N, n, gravity, precision):
     (2, 4, 10, 64, 0.0), (2, 7, 40, 64, 0.0), (2, 4, 60, 32, 0.0), (2, 7, 30, 64, 0.02), (2, 4, 20, 32, 0.02),
     (3, 3, 9, 64, 0.0), (3, 4, 14, 32, 0.0), (3, 4, 8, 64, 0.0), (3, 5, 8, 64, 0.0), (3, 7, 8, 64, 0.0),
     (3, 7, 8, 32, 0.0), (3, 10, 4, 64, 0.0), (3, 3, 4, 64, 0.02), (3, 3, 17, 32, 0.02), (3, 5, 4, 32, 0.02),
-    (3, 7, 10, 64, 0.02)])
+    (3, 7, 10, 64, 0.02), (3, 5, 10, 32, 0.02), (3, 6, 4, 64, 0.02)])
 def test_run_equals_stage_calls(dim, N, n, precision, visc):
     m, Q, dt = case(dim, N, n)
     a, b = (solver(m, Q, precision, dict(dg.WORKLOAD_PHYS, visc=visc)) for _ in range(2))
