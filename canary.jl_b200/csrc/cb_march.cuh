@@ -104,6 +104,17 @@ __device__ __forceinline__ double ld_here(const double *p) {
   return v;
 }
 
+// Pointers that the compiler cannot take for read-only parameters, whose loads it
+// otherwise schedules over the whole kernel at the price of registers (us a step
+// without / with: viscous FP64 N=2 33^3 1520 / 1478, N=5 25^3 4180 / 4113, Euler FP64 N=8
+// 17^3 1699 / 1682).
+template <typename... P>
+__device__ __forceinline__ void here_pointers(P *&...ptr) {
+  int64_t zero;
+  asm volatile("mov.s64 %0, 0;" : "=l"(zero)::"memory");
+  ((void)(ptr += zero), ...);
+}
+
 // D by rows i (DT[i][m] = D[m + Nq i]) and by rows m (DZ[m][i]).
 template <int Nq, int RS, int THREADS, typename T>
 __device__ __forceinline__ void march_load_D(T *DT, T *DZ, const T *__restrict__ D) {
@@ -203,6 +214,7 @@ __global__ void __launch_bounds__(March<Nq, T>::THREADS,
   T *DT = reinterpret_cast<T *>(smem_raw + C::OFF_DT), *DZ = reinterpret_cast<T *>(smem_raw + C::OFF_DZ);
   T *PL = reinterpret_cast<T *>(smem_raw + C::OFF_P);
   T *FF = reinterpret_cast<T *>(smem_raw + C::OFF_FF);
+  here_pointers(a.Qin, a.Qout, a.rhs, a.gq);
   const int tid = threadIdx.x, el = tid / N2, ij = tid % N2, i = ij % Nq, j = ij / Nq;
   const int64_t e0 = a.ebeg + (int64_t)blockIdx.x * EPB, e = e0 + el;
   const bool act = el < EPB && e < a.eend;
@@ -559,6 +571,7 @@ __global__ void __launch_bounds__(March<Nq, T>::THREADS, March<Nq, T>::blocks_fo
   using V = typename Vec16<T>::type;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T *DS = reinterpret_cast<T *>(smem_raw), *S = reinterpret_cast<T *>(smem_raw + C::OFF_S);
+  here_pointers(A.Qin, A.gq);
   const int tid = threadIdx.x, el = tid / N2, ab = tid % N2;
   const int64_t e0 = A.ebeg + (int64_t)blockIdx.x * EPB;
   LineCtx<Nq, T> c;
