@@ -48,7 +48,9 @@ inline cudaError_t launch_stage_kernel(void (*kernel)(K...), unsigned grid, int 
   c.stream = st;
   c.attrs = &at;
   c.numAttrs = 1;
-  return cudaLaunchKernelEx(&c, kernel, K(args)...);
+  const cudaError_t e = cudaLaunchKernelEx(&c, kernel, K(args)...);
+  if (e != cudaSuccess) cudaGetLastError();  // returned here: not left for the next launch's check
+  return e;
 }
 
 // Mirror of the public cb_phys.
