@@ -7,9 +7,9 @@
 // consecutive elements; a thread owns nodes t, t+THREADS, ... of that group.
 // The element-local stage is: pointwise fluxes -> shared memory ->
 // tensor-product contraction with D -> face fluxes into a shared face buffer
-// -> per-node accumulation in face order -> update.  All sums run in the
-// same order as the reference CPU loops so that FP64 results agree to
-// round-off.
+// -> per-node accumulation in face order -> update, sums in the order of the
+// reference CPU loops.  The stages by grid lines (cb_march.cuh) add the terms of
+// a line where they are formed.  FP64 results of all agree to round-off.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -27,7 +27,8 @@ namespace cb {
 // directly follows a pass of the same solve is programmatic (chained): what else
 // may precede it in the stream can write the geometry.  The pointers depend
 // on the instruction: loads from them (read-only data to the compiler) cannot be
-// moved above it.  Both instructions do nothing in a plain launch.
+// moved above it.  Both instructions do nothing in a plain launch.  Which chained
+// launches are programmatic: Launch::chain_pays.
 template <typename... P>
 __device__ __forceinline__ void grid_wait(P *&...ptr) {
   int64_t zero;

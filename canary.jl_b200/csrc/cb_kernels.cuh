@@ -910,7 +910,7 @@ struct Launch {
     // 10.2 / 11.3, 20^3 46.6 / 44.3; N=5 7^3 5.2 / 6.1, 10^3 9.8 / 9.1; N=7 5^3 5.3 / 6.2, 8^3
     // 15.4 / 11.2; N=10 5^3 13.7 / 14.4; FP32 N=3 10^3 2.8 / 3.0, 15^3 4.8 / 4.5; N=6 6^3 4.5 /
     // 6.6, 9^3 8.3 / 8.3; N=9 4^3 6.0 / 6.7, 6^3 9.8 / 8.5).
-    if constexpr (DIM == 3 && Nq >= (sizeof(T) == 4 ? 4 : 5)) {
+    if constexpr (DIM == 3 && march_volume_built(Nq, sizeof(T))) {
       constexpr int GROUPED_BLOCKS = Nq >= 9 ? 1 : Nq == 5 ? 8 : 3;
       if (grid(nelem) > GROUPED_BLOCKS * num_sms()) return march_volume<T>(Nq, rhs, Q, vgeo, D, nelem, p, st);
     }
@@ -947,7 +947,7 @@ struct Launch {
   // element per SM keep the grouped stage, whose block spreads an element over 512
   // threads (5^3, us a step, grouped / march: FP64 N=8 52 / 83, N=9 65 / 84, N=10 100 /
   // 116, FP32 N=10 64 / 75; 6^3: 99 / 106, 125 / 118, 196 / 174, 106 / 97).
-  static constexpr bool MARCH = DIM == 3 && (Nq >= 11 || (Nq >= 9 && sizeof(T) == 8));
+  static constexpr bool MARCH = DIM == 3 && march_inviscid(Nq, sizeof(T));
   // Default stage kernel per shape, from B200 timings of one mesh (ms per
   // step, warped 3-D cubes of 7-17 M nodes; pipelined CUDA-core / grouped /
   // lean): FP64 N=3 3.66 / 3.34 / 2.76, N=4 4.95 / 4.20 / 3.78, N=5 2.37 /
@@ -959,6 +959,8 @@ struct Launch {
   // first figure is the grouped stage as well).  N=2, 6.1 M nodes: FP64 4.30 /
   // 3.18 / 3.42, FP32 1.83 / 1.33 / 1.64; N=1: FP64 4.52 / 3.30 / 3.90, FP32
   // 2.87 / 1.36 / 2.43.  3-D N=7 runs the tensor-core stage in both precisions.
+  // (N=3 to 9: timed before the stages formed contravariant fluxes directly, which
+  // took 1 to 10 % off each and kept their order.)
   static constexpr int DEFAULT_KERNEL =
       MARCH         ? 5
       : MMA_DEFAULT ? 2
@@ -982,7 +984,9 @@ struct Launch {
   static constexpr bool EARLY_OK = C::NPT == 1 && !MARCH && (DIM == 2 || DEFAULT_KERNEL == 3);
   // (us a stage, stages in a row on one solver: FP32 3-D N=3 8^3 4.9 -> 3.0, 12^3
   // 6.4 -> 5.6, N=4 8^3 5.9 -> 4.4, N=6 6^3 6.8 -> 5.3, 2-D N=4 48^2 5.7 -> 3.2;
-  // FP64 2-D N=4 10^2 4.9 -> 2.9, but N=7 32^2 4.5 at one block, 5.6 at two)
+  // FP64 2-D N=4 10^2 4.9 -> 2.9, but N=7 32^2 4.5 at one block, 5.6 at two; 2-D
+  // against the pipelined stage, time ratios over N=1 to 10: 10^2 FP64 0.57 to 0.84,
+  // FP32 0.56 to 0.93, 32^2 FP32 0.55 to 0.89, 48^2 FP32 at N <= 7 0.56 to 0.96)
   static constexpr int EARLY_BLOCKS = sizeof(T) == 4 ? 4 : 1;
   static bool small_mesh(int64_t nelem) {
     return EARLY_OK && (nelem + C::EPB - 1) / C::EPB <= (int64_t)EARLY_BLOCKS * num_sms();
@@ -1143,7 +1147,8 @@ struct Launch {
       cudaError_t err = prep(k_stage<DIM, Nq, T>, sm);
       if (err != cudaSuccess) return err;
       // (plain up to a wave: the next stage's blocks would crowd onto the SMs that
-      // have room, FP32 N=4 10^3: 9.5 us a stage against 7.6)
+      // have room, FP32 N=4 10^3: 9.5 us a stage against 7.6; from 2000 blocks on,
+      // FP32 N=2 to 6, both within 1 %)
       return launch_stage_kernel(k_stage<DIM, Nq, T>, (unsigned)groups, C::THREADS, sm, st, chained && groups > 8 * num_sms(),
                                  Qin, Qout, rhs, vgeo, sgeo, nbr, D, nelem, p, qref, rka, rkbdt, status, ebeg);
     }

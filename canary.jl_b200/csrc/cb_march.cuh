@@ -5,8 +5,10 @@
 // made, straight into the line's accumulators: no exchange, and D is read
 // uniformly by the block.  (The node-owner stages read Nq flux values per node,
 // field and direction from shared memory; they are bound by that pipe.)  Both
-// kernels below use only plain and cp.async accesses of single values, so there
-// is no rule on the alignment of arrays or element slabs.
+// kernels below read the state, the carry and the geometry by plain and cp.async
+// accesses of single values, so there is no rule on the alignment of the caller's
+// arrays or of element slabs; the neighbour codes (read in pairs) and the gradient
+// records (in 16-byte vectors) are the solver's own allocations.
 //
 // k_march_stage: the fused stage, inviscid or (VISC) with the viscous flux.  The
 // thread (i, j) owns the ζ line (i, j, 0..N) and the block marches through the
@@ -793,20 +795,24 @@ struct MarchLaunch {
     return cudaGetLastError();
   }
   static cudaError_t stage(bool visc, const MarchArgs<T> &a, const PhysT<T> &p, cudaStream_t st) {
-    return visc ? launch(k_march_stage<Nq, T, true>, M::smem_stage(), a, p, st)
-                : launch(k_march_stage<Nq, T, false>, M::smem_stage(), a, p, st);
+    if (visc) return launch(k_march_stage<Nq, T, true>, M::smem_stage(), a, p, st);
+    if constexpr (march_inviscid(Nq, sizeof(T))) return launch(k_march_stage<Nq, T, false>, M::smem_stage(), a, p, st);
+    return cudaErrorNotSupported;
   }
   static cudaError_t volume(T *rhs, const T *Q, const T *vgeo, const T *D, int64_t nelem, const PhysT<T> &p,
                             cudaStream_t st) {
-    const int64_t g = (nelem + M::EPB - 1) / M::EPB;
-    if (g <= 0) return cudaSuccess;
-    if (M::smem_volume() > 48 * 1024) {
-      const cudaError_t e = cudaFuncSetAttribute(k_march_volume<Nq, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)M::smem_volume());
-      if (e != cudaSuccess) return e;
+    if constexpr (march_volume_built(Nq, sizeof(T))) {
+      const int64_t g = (nelem + M::EPB - 1) / M::EPB;
+      if (g <= 0) return cudaSuccess;
+      if (M::smem_volume() > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(k_march_volume<Nq, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)M::smem_volume());
+        if (e != cudaSuccess) return e;
+      }
+      k_march_volume<Nq, T><<<(unsigned)g, M::THREADS, M::smem_volume(), st>>>(rhs, Q, vgeo, D, nelem, p);
+      return cudaGetLastError();
     }
-    k_march_volume<Nq, T><<<(unsigned)g, M::THREADS, M::smem_volume(), st>>>(rhs, Q, vgeo, D, nelem, p);
-    return cudaGetLastError();
+    return cudaErrorNotSupported;
   }
   static cudaError_t grad(const MarchArgs<T> &a, const PhysT<T> &p, cudaStream_t st) {
     return launch(k_line_grad<Nq, T>, M::smem_grad(), a, p, st);

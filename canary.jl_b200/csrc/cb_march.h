@@ -25,6 +25,11 @@ struct MarchArgs {
   unsigned *status;
 };
 
+// The shapes whose inviscid stage and whose volume integral are built (where
+// Launch chooses them); the viscous passes are built for every order.
+constexpr bool march_inviscid(int Nq, size_t w) { return Nq >= 11 || (Nq >= 9 && w == 8); }
+constexpr bool march_volume_built(int Nq, size_t w) { return Nq >= (w == 4 ? 4 : 5); }
+
 // Fused stage of order Nq - 1 (visc: the second viscous pass) and the
 // gradient pass.
 template <typename T>

@@ -99,8 +99,9 @@ struct PipeMT {
   // stage; four blocks at 64 registers spill and take 0.637 ms)
   // (FP32 with the prefetch one group ahead: 0.567 ms, the same)
   // PFD = -2: one group ahead, at the middle of the iteration (FP32 with its
-  // half-size plan: 2.54 ms per step at 32^3 against 2.60; FP64, whose blocks
-  // then hold too much of L2: 5.21 against 4.86)
+  // half-size plan, us a step: 14^3 231 against 244, 16^3 334 / 346, 18^3 473 / 488,
+  // 12^3 and below the same; 32^3 within the noise of a hot card; FP64, whose blocks
+  // then hold too much of L2: 32^3 5.21 against 4.86 ms)
   static constexpr int MINB = sizeof(T) == 8 ? 2 : 3, PFD = sizeof(T) == 8 ? -1 : -2;
   // whether this stage is the default of its shape (the faster on B200 at
   // 32^3 hexes: FP64 0.974 ms per stage against 1.17 ms for the CUDA-core

@@ -157,7 +157,9 @@ int cb_flux_div(int dim, int N, double *rhs, const double *gradQ,
  *                 once into solver-owned FP32 copies.
  * The solver owns its scratch (a second state buffer for the double-buffered
  * stage, compact int32 face-neighbour tables built from vmapM/vmapP, the
- * gradient arrays of the viscous form and the captured CUDA graph). */
+ * gradient arrays of the viscous form and the captured CUDA graph).  The face
+ * maps are read once, at creation; viscous 3-D N >= 8 also takes maps that are
+ * not conforming, and reads those at every step. */
 typedef struct cb_solver cb_solver;
 
 int cb_solver_create(cb_solver **out, int dim, int N, int precision,
@@ -182,7 +184,8 @@ int cb_solver_set_offset(cb_solver *s, const double *qref);
 int cb_solver_sums(cb_solver *s, double *out_host);
 /* Enqueue on the solver's stream a copy of its status bits (bit 2:
  * non-finite state) into *out_host (page-locked memory for an asynchronous
- * copy); the value is valid once the stream has reached the copy. */
+ * copy); the value is valid once the stream has reached the copy.  Viscous 3-D
+ * N >= 8 does not raise bit 2. */
 int cb_solver_status_async(cb_solver *s, unsigned *out_host);
 /* Stage kernel: 0 = the default for the mesh, 1 = the CUDA-core stages
  * (pipelined bulk-copy staging where the plan fits), 2 = the tensor-core
@@ -262,8 +265,8 @@ int cb_solver_unpack_faces(cb_solver *s, int what, const int64_t *codes, int64_t
  * stage for those elements, half = 1 for the others (once the ghosts of the
  * state the stage reads are filled) and then makes the other buffer
  * current; a stage split this way equals cb_solver_stage bit for bit.
- * Inviscid form, shapes whose stage runs over element ranges (the pipelined,
- * lean and tensor-core stages); CB_ERR_UNSUPPORTED otherwise. */
+ * Inviscid form, 16-byte aligned arrays, every order but 3-D N=10 in FP64;
+ * CB_ERR_UNSUPPORTED otherwise. */
 int cb_solver_set_split(cb_solver *s, int64_t ninterior);
 int cb_solver_stage_split(cb_solver *s, int stage, double dt, int half, void **next_in);
 
