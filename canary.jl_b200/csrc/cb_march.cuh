@@ -697,89 +697,16 @@ __global__ void __launch_bounds__(March<Nq, T>::THREADS, March<Nq, T>::blocks_fo
     __syncthreads();  // the sums are rewritten for the next direction; the next field
     copy_field(3 * cc + 5);
   }
-}
-
-// Density gradient: ∂_c ρ = MJI (-Σ_r Dᵀ(MJ ξ_r,c ρ) + Σ_f sMJ n_c (ρ⁻ + ρ⁺)/2), a
-// thread a node, the nine products MJ ξ_r,c ρ of the block's elements in shared
-// memory.  Not on a step's path: it runs where a packed gradient is asked for.
-template <int Nq, typename T>
-struct DensityPlan {
-  using C = Cfg<3, Nq>;
-  static constexpr size_t smem() { return sizeof(T) * (Nq * Nq + 9 * (size_t)C::SLOTS); }
-};
-template <int Nq, typename T>
-__global__ void __launch_bounds__(Cfg<3, Nq>::THREADS)
-    k_density_grad(const T *__restrict__ Q, T *__restrict__ out, const T *__restrict__ vgeo, const T *__restrict__ sgeo,
-                   const int32_t *__restrict__ nbr, const T *__restrict__ D, int64_t nelem, T rho_ref) {
-  using C = Cfg<3, Nq>;
-  constexpr int Np = C::Np, N2 = Nq * Nq, SP = C::SLOTS, NS = 5, NVG = 14, NSG = 5, IR = 3, MJF = 9, MJIF = 10;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T *h = reinterpret_cast<T *>(smem_raw), *Ds = h + 9 * SP;  // [9][SP]: direction r of component c at r + 3 c
-  const int64_t e0 = (int64_t)blockIdx.x * C::EPB;
-  for (int t = threadIdx.x; t < N2; t += C::THREADS) Ds[t] = D[t];
+  // (read again at the end: a store in the loop above, also one never taken, cost FP32
+  // N=5 20^3 3 % of a step, 1111 -> 1148 us)
+  if (A.rho && c.act)
 #pragma unroll
-  for (int u = 0; u < C::NPT; ++u) {
-    const int slot = threadIdx.x + u * C::THREADS, n = slot % Np;
-    const int64_t e = e0 + slot / Np;
-    if (slot < SP && e < nelem) {
-      const T *vg = vgeo + e * (Np * NVG) + n;
-      const T v = vg[Np * MJF] * (Q[e * (Np * NS) + Np * IR + n] + rho_ref);
-#pragma unroll
-      for (int f = 0; f < 9; ++f) h[f * SP + slot] = v * vg[Np * f];
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int u = 0; u < C::NPT; ++u) {
-    const int slot = threadIdx.x + u * C::THREADS, n = slot % Np;
-    const int64_t e = e0 + slot / Np;
-    if (slot >= SP || e >= nelem) continue;
-    const int i = n % Nq, j = n / Nq % Nq, k = n / N2;
-    const T *hl = h + (slot - n);
-    T a[3] = {T(0), T(0), T(0)};
-#pragma unroll
-    for (int m = 0; m < Nq; ++m) {
-      const T di = Ds[m + Nq * i], dj = Ds[m + Nq * j], dk = Ds[m + Nq * k];
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-        a[c] -= di * hl[3 * c * SP + m + Nq * j + N2 * k] + dj * hl[(3 * c + 1) * SP + i + Nq * m + N2 * k] +
-                dk * hl[(3 * c + 2) * SP + i + Nq * j + N2 * m];
-    }
-    const T own = Q[e * (Np * NS) + Np * IR + n] + rho_ref;
-    auto face = [&](int f, int fn) {
-      const int32_t code = nbr[f + 6 * e];
-      const T *sg = sgeo + NSG * (fn + (int64_t)N2 * (f + 6 * e));
-      const T other =
-          code < 0 ? own : Q[face_node<3, Nq>(code & 7, fn) + Np * (IR + NS * (int64_t)(code >> 3))] + rho_ref;
-      const T w = sg[3] * (T(0.5) * (own + other));
-#pragma unroll
-      for (int c = 0; c < 3; ++c) a[c] += w * sg[c];
-    };
-    if (i == 0 || i == Nq - 1) face(i == 0 ? 0 : 1, j + Nq * k);
-    if (j == 0 || j == Nq - 1) face(j == 0 ? 2 : 3, i + Nq * k);
-    if (k == 0 || k == Nq - 1) face(k == 0 ? 4 : 5, i + Nq * j);
-    const T mji = vgeo[e * (Np * NVG) + n + Np * MJIF];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) out[e * (3 * Np) + n + Np * c] = a[c] * mji;
-  }
+    for (int x = 0; x < Nq; ++x) A.rho[c.e * Np + ab + N2 * x] = c.Q[ab + N2 * x + Np * IR] + qr[IR];
 }
 
 template <int Nq, typename T>
 struct MarchLaunch {
   using M = March<Nq, T>;
-  static cudaError_t density(const T *Q, T *out, const T *vgeo, const T *sgeo, const int32_t *nbr, const T *D,
-                             int64_t nelem, T rho_ref, cudaStream_t st) {
-    using C = Cfg<3, Nq>;
-    constexpr size_t smem = DensityPlan<Nq, T>::smem();
-    if (nelem == 0) return cudaSuccess;
-    if (smem > 48 * 1024) {
-      const cudaError_t e = cudaFuncSetAttribute(k_density_grad<Nq, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return e;
-    }
-    k_density_grad<Nq, T><<<(unsigned)((nelem + C::EPB - 1) / C::EPB), C::THREADS, smem, st>>>(Q, out, vgeo, sgeo, nbr, D,
-                                                                                              nelem, rho_ref);
-    return cudaGetLastError();
-  }
   template <typename K>
   static cudaError_t launch(K kernel, size_t smem, const MarchArgs<T> &a, const PhysT<T> &p, cudaStream_t st) {
     const int64_t g = (a.eend - a.ebeg + M::EPB - 1) / M::EPB;
@@ -851,17 +778,5 @@ struct MarchLaunch {
         &MarchLaunch<6, T_>::grad, &MarchLaunch<7, T_>::grad, &MarchLaunch<8, T_>::grad, &MarchLaunch<9, T_>::grad, \
         &MarchLaunch<10, T_>::grad, &MarchLaunch<11, T_>::grad};                                                    \
     return Nq < 2 || Nq > 11 ? cudaErrorInvalidValue : f[Nq - 2](a, p, st);                                         \
-  }                                                                                                                 \
-  template <>                                                                                                       \
-  cudaError_t density_gradient<T_>(int Nq, const T_ *Q, T_ *out, const T_ *vgeo, const T_ *sgeo,                    \
-                                   const int32_t *nbr, const T_ *D, int64_t nelem, T_ rho_ref, cudaStream_t st) {   \
-    static cudaError_t (*const f[])(const T_ *, T_ *, const T_ *, const T_ *, const int32_t *, const T_ *, int64_t, \
-                                    T_, cudaStream_t) = {                                                           \
-        &MarchLaunch<2, T_>::density, &MarchLaunch<3, T_>::density, &MarchLaunch<4, T_>::density,                   \
-        &MarchLaunch<5, T_>::density, &MarchLaunch<6, T_>::density, &MarchLaunch<7, T_>::density,                   \
-        &MarchLaunch<8, T_>::density, &MarchLaunch<9, T_>::density, &MarchLaunch<10, T_>::density,                  \
-        &MarchLaunch<11, T_>::density};                                                                             \
-    return Nq < 2 || Nq > 11 ? cudaErrorInvalidValue                                                                \
-                             : f[Nq - 2](Q, out, vgeo, sgeo, nbr, D, nelem, rho_ref, st);                           \
   }                                                                                                                 \
   }

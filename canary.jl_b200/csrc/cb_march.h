@@ -23,6 +23,7 @@ struct MarchArgs {
   Offs<T, 5> qref;
   T rka, rkbdt;
   unsigned *status;
+  T *rho = nullptr;  // where given, the gradient pass leaves the density of its input there, [element][Np]
 };
 
 // The shapes whose inviscid stage and whose volume integral are built (where
@@ -40,10 +41,5 @@ cudaError_t march_volume(int Nq, T *rhs, const T *Q, const T *vgeo, const T *D, 
                          cudaStream_t st);
 template <typename T>
 cudaError_t march_grad(int Nq, const MarchArgs<T> &a, const PhysT<T> &p, cudaStream_t st);
-// Density gradient (Np, 3, nelem) of the state Q, which the records leave out (it
-// does not enter the viscous flux): for callers who take the whole gradient.
-template <typename T>
-cudaError_t density_gradient(int Nq, const T *Q, T *out, const T *vgeo, const T *sgeo, const int32_t *nbr, const T *D,
-                             int64_t nelem, T rho_ref, cudaStream_t st);
 
 }  // namespace cb

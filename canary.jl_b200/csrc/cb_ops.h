@@ -58,9 +58,10 @@ struct Ops {
   cudaError_t (*cons_sums)(const T *, const T *, int64_t, int, const Offs<double, 5> &, double *, int,
                            cudaStream_t);
   // fused viscous passes over one mesh: pass 0 (gradient) or 1 (stage +
-  // update); the last arguments are the kernel (1, 3 or 5) and whether the
-  // stream's preceding launch is a pass of the same solve
-  cudaError_t (*ns_pass)(int, const BDesc<T> &, T *, int64_t, const PhysT<T> &, T, T, cudaStream_t, int, int);
+  // update).  Arguments: the gradient, where the gradient pass of kernel 5 leaves
+  // the density (or null), ..., the kernel (1, 3 or 5) and whether the stream's
+  // preceding launch is a pass of the same solve
+  cudaError_t (*ns_pass)(int, const BDesc<T> &, T *, T *, int64_t, const PhysT<T> &, T, T, cudaStream_t, int, int);
   // whether the viscous form of this order has stage calls, ghosts and state
   // offsets (every 2-D order, 3-D N <= 7)
   bool ns_stage_form;

@@ -41,10 +41,11 @@ struct cb_solver {
   // form the gradient buffer is in: 0 not written yet, 1 (Np, nstate, dim,
   // elements), 2 records (grad_at)
   int grad_form = 0;
-  // records: the state (Q or the twin, the input of the last gradient pass)
-  // whose density gradient the buffer still lacks; no pass reads it, so it is
-  // formed when the gradient is packed or that state is about to change
-  const void *rho_src = nullptr;
+  // 3-D: the density of the state that the last gradient pass by grid lines read,
+  // [element][Np], ghosts included.  No pass reads the density gradient: while
+  // rho_live is set, that of an own element is formed from rho where a caller packs it
+  void *rho = nullptr;
+  bool rho_live = false;
   cb_phys phys{};
   cudaStream_t stream = nullptr;
   bool own_stream = false;
@@ -92,6 +93,10 @@ int kernel_of(const cb_solver *s) {
 // the state ping-pongs between Q and Qalt (two steps per graph)
 bool pingpong(const cb_solver *s) { return s->phys.visc <= 0 || fused_visc(s); }
 
+bool records_wanted(const cb_solver *s);
+template <typename T>
+cudaError_t ghost_density(cb_solver *s, const T *Q);
+
 // One step; chained: the stream's preceding launch is the step before it.
 template <typename T>
 cudaError_t enqueue_step(cb_solver *s, double dt, bool from_user, bool chained) {
@@ -114,11 +119,13 @@ cudaError_t enqueue_step(cb_solver *s, double dt, bool from_user, bool chained) 
     for (int st = 0; st < 5 && e == cudaSuccess; ++st) {
       I.Q[0] = a;
       I.Q[1] = b;
-      if ((e = o->ns_pass(0, I, (T *)s->gradQ, s->nelem, p, T(0), T(0), s->stream, kernel_of(s),
+      T *rho = st == 4 && records_wanted(s) ? (T *)s->rho : nullptr;  // of the last gradient
+      if (rho && (e = ghost_density<T>(s, a)) != cudaSuccess) break;
+      if ((e = o->ns_pass(0, I, (T *)s->gradQ, rho, s->nelem, p, T(0), T(0), s->stream, kernel_of(s),
                           chained || st)) != cudaSuccess)
         break;
-      e = o->ns_pass(1, I, (T *)s->gradQ, s->nelem, p, T(RKA[(st + 1) % 5]), T(RKB[st] * dt), s->stream, kernel_of(s),
-                     1);
+      e = o->ns_pass(1, I, (T *)s->gradQ, nullptr, s->nelem, p, T(RKA[(st + 1) % 5]), T(RKB[st] * dt), s->stream,
+                     kernel_of(s), 1);
       T *t = a;
       a = b;
       b = t;
@@ -210,27 +217,9 @@ int64_t nodes(const cb_solver *s) {
 }
 unsigned blocks_for(int64_t total) { return (unsigned)std::min<int64_t>((total + 255) / 256, 148 * 16); }
 
-// Density gradient of the state `src` into the records' density part.
-template <typename T>
-cudaError_t density_gradient(cb_solver *s, const void *src) {
-  s->rho_src = nullptr;
-  return cb::density_gradient<T>(s->N + 1, (const T *)src, (T *)s->gradQ + GREC * nodes(s) * (s->nelem + s->nghost),
-                                 (const T *)s->vgeo, (const T *)s->sgeo, s->nbr, (const T *)s->D, s->nelem,
-                                 T(s->qref[3]), s->stream);
-}
-cudaError_t density_gradient(cb_solver *s, const void *src) {
-  return s->prec == 64 ? density_gradient<double>(s, src) : density_gradient<float>(s, src);
-}
-// the whole gradient; with `about_to_change`, only if it lacks that state's
-cudaError_t complete_gradient(cb_solver *s, const void *about_to_change = nullptr) {
-  if (!s->rho_src || (about_to_change && about_to_change != s->rho_src)) return cudaSuccess;
-  return density_gradient(s, s->rho_src);
-}
 // bring the state back into the caller's Q after an odd number of stages
 cudaError_t settle(cb_solver *s) {
   if (!s->cur) return cudaSuccess;
-  const cudaError_t e = complete_gradient(s, s->Q);
-  if (e != cudaSuccess) return e;
   s->cur = 0;
   return cudaMemcpyAsync(s->Q, s->Qalt, state_bytes(s), cudaMemcpyDeviceToDevice, s->stream);
 }
@@ -244,15 +233,77 @@ __host__ __device__ __forceinline__ T *grad_at(T *gq, int64_t Np, int64_t nall, 
                  : gq + GREC * (node + Np * el) + 4 * d + (s5 == 4 ? 3 : s5);
 }
 
+// Density gradient of an own element from the density rho (null: not kept, the
+// records hold the gradient itself).
+template <typename T>
+struct DensityOf {
+  const T *rho, *vgeo, *sgeo, *D;
+  const int32_t *nbr;
+  int64_t nown;
+  int Nq;
+};
+template <typename T>
+DensityOf<T> density_of(const cb_solver *s) {
+  return {s->rho_live ? (const T *)s->rho : nullptr, (const T *)s->vgeo, (const T *)s->sgeo, (const T *)s->D, s->nbr,
+          s->nelem, s->N + 1};
+}
+// Component c at a node: MJI (-Σ_r Dᵀ(MJ ξ_r,c ρ) + Σ_f sMJ n_c (ρ⁻ + ρ⁺)/2).
+template <typename T>
+__device__ T density_gradient(const DensityOf<T> &d, int64_t el, int node, int c) {
+  const int Nq = d.Nq, N2 = Nq * Nq, Np = N2 * Nq;
+  const int pos[3] = {node % Nq, node / Nq % Nq, node / N2}, step[3] = {1, Nq, N2};
+  const T *vg = d.vgeo + el * (Np * 14), *rho = d.rho + el * Np;
+  T a = T(0);
+#pragma unroll
+  for (int r = 0; r < 3; ++r) {
+    const int first = node - pos[r] * step[r];
+    for (int m = 0; m < Nq; ++m) {
+      const int l = first + m * step[r];
+      a -= d.D[m + Nq * pos[r]] * (vg[l + Np * 9] * vg[l + Np * (r + 3 * c)] * rho[l]);
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < 3; ++r) {
+    if (pos[r] != 0 && pos[r] != Nq - 1) continue;
+    const int f = 2 * r + (pos[r] != 0), fn = r == 0 ? pos[1] + Nq * pos[2] : pos[0] + Nq * pos[r == 1 ? 2 : 1];
+    const int32_t code = d.nbr[f + 6 * el];
+    const T other = code < 0 ? rho[node] : d.rho[face_node_rt<3>(Nq, code & 7, fn) + Np * (int64_t)(code >> 3)];
+    const T *sg = d.sgeo + 5 * (fn + (int64_t)N2 * (f + 6 * el));
+    a += sg[c] * (sg[3] * (T(0.5) * (rho[node] + other)));
+  }
+  return a * vg[node + Np * 10];
+}
+// Gradient component d of field s5 as a caller reads it.
+template <typename T>
+__device__ __forceinline__ T grad_value(T *gq, int64_t Np, int64_t nall, int64_t el, int64_t node, int s5, int d,
+                                        const DensityOf<T> &rho) {
+  if (s5 == 3 && rho.rho && el < rho.nown) return density_gradient(rho, el, (int)node, d);
+  return *grad_at(gq, Np, nall, el, node, s5, d);
+}
+
+// The density of the ghosts, beside that which the gradient pass leaves.
+template <typename T>
+__global__ void k_ghost_density(const T *__restrict__ Q, T *__restrict__ rho, int64_t Np, int64_t first, int64_t n, T ref) {
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n * Np; t += (int64_t)gridDim.x * blockDim.x)
+    rho[first * Np + t] = Q[(5 * (first + t / Np) + 3) * Np + t % Np] + ref;
+}
+template <typename T>
+cudaError_t ghost_density(cb_solver *s, const T *Q) {
+  if (!s->nghost) return cudaSuccess;
+  k_ghost_density<T><<<blocks_for(s->nghost * nodes(s)), 256, 0, s->stream>>>(Q, (T *)s->rho, nodes(s), s->nelem, s->nghost,
+                                                                              T(s->qref[3]));
+  return cudaGetLastError();
+}
+
 // The gradient between its two forms: `plain` is (Np, 5, 3, nall).
 template <typename T>
-__global__ void k_grad_form(bool to_records, T *__restrict__ plain, T *__restrict__ rec, int64_t Np, int64_t nall) {
+__global__ void k_grad_form(bool to_records, T *__restrict__ plain, T *__restrict__ rec, int64_t nall, DensityOf<T> rho) {
+  const int64_t Np = (int64_t)rho.Nq * rho.Nq * rho.Nq;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < 15 * Np * nall; t += (int64_t)gridDim.x * blockDim.x) {
     const int64_t el = t / (15 * Np);
     const int c = (int)(t / Np % 15);
-    T *r = grad_at(rec, Np, nall, el, t % Np, c % 5, c / 5);
-    if (to_records) *r = plain[t];
-    else plain[t] = *r;
+    if (to_records) *grad_at(rec, Np, nall, el, t % Np, c % 5, c / 5) = plain[t];
+    else plain[t] = grad_value(rec, Np, nall, el, t % Np, c % 5, c / 5, rho);
   }
 }
 // Bring the gradient buffer into the form that the kernel choice works with
@@ -260,8 +311,7 @@ __global__ void k_grad_form(bool to_records, T *__restrict__ plain, T *__restric
 cudaError_t adopt_form(cb_solver *s) {
   const bool want = records_wanted(s);
   if (records(s) == want) return cudaSuccess;
-  cudaError_t e = complete_gradient(s);
-  if (e != cudaSuccess) return e;
+  cudaError_t e;
   const int64_t Np = nodes(s), nall = s->nelem + s->nghost;
   const size_t bytes = (s->prec == 64 ? 8 : 4) * (size_t)(15 * Np * nall);
   void *old = nullptr;
@@ -269,10 +319,13 @@ cudaError_t adopt_form(cb_solver *s) {
   if ((e = cudaMemcpyAsync(old, s->gradQ, bytes, cudaMemcpyDeviceToDevice, s->stream)) == cudaSuccess) {
     void *plain = want ? old : s->gradQ, *rec = want ? s->gradQ : old;
     if (s->prec == 64)
-      k_grad_form<double><<<blocks_for(15 * Np * nall), 256, 0, s->stream>>>(want, (double *)plain, (double *)rec, Np, nall);
+      k_grad_form<double><<<blocks_for(15 * Np * nall), 256, 0, s->stream>>>(want, (double *)plain, (double *)rec, nall, density_of<double>(s));
     else
-      k_grad_form<float><<<blocks_for(15 * Np * nall), 256, 0, s->stream>>>(want, (float *)plain, (float *)rec, Np, nall);
-    if ((e = cudaGetLastError()) == cudaSuccess) s->grad_form = want ? 2 : 1;
+      k_grad_form<float><<<blocks_for(15 * Np * nall), 256, 0, s->stream>>>(want, (float *)plain, (float *)rec, nall, density_of<float>(s));
+    if ((e = cudaGetLastError()) == cudaSuccess) {
+      s->grad_form = want ? 2 : 1;
+      s->rho_live = false;  // (it is stored with the others)
+    }
   }
   const cudaError_t ef = cudaFreeAsync(old, s->stream);
   return e == cudaSuccess ? ef : e;
@@ -281,7 +334,6 @@ cudaError_t adopt_form(cb_solver *s) {
 cudaError_t adopt_form_anew(cb_solver *s) {
   if (s->nghost) return adopt_form(s);
   s->grad_form = records_wanted(s) ? 2 : 1;
-  s->rho_src = nullptr;
   return cudaSuccess;
 }
 
@@ -306,14 +358,18 @@ cudaError_t enqueue_pass(cb_solver *s, int st, double dt, int pass) {
     I.status = visc_status(s);
     I.dt = dt;
     for (int k = 0; k < 5; ++k) I.qref[k] = T(s->qref[k]);
-    cudaError_t e = pass == 0 ? adopt_form_anew(s) : adopt_form(s);
+    const cudaError_t e = pass == 0 ? adopt_form_anew(s) : adopt_form(s);
     if (e != cudaSuccess) return e;
     if (pass == 0) {
-      s->rho_src = records(s) ? a : nullptr;
-      return o->ns_pass(0, I, (T *)s->gradQ, s->nelem, p, T(0), T(0), s->stream, kernel_of(s), 0);
+      if (records(s)) {
+        s->rho_live = true;
+        const cudaError_t eg = ghost_density<T>(s, a);
+        if (eg != cudaSuccess) return eg;
+      }
+      return o->ns_pass(0, I, (T *)s->gradQ, (T *)s->rho, s->nelem, p, T(0), T(0), s->stream, kernel_of(s), 0);
     }
-    if ((e = complete_gradient(s, b)) != cudaSuccess) return e;
-    return o->ns_pass(1, I, (T *)s->gradQ, s->nelem, p, T(RKA[(st + 1) % 5]), T(RKB[st] * dt), s->stream, kernel_of(s), 0);
+    return o->ns_pass(1, I, (T *)s->gradQ, nullptr, s->nelem, p, T(RKA[(st + 1) % 5]), T(RKB[st] * dt), s->stream,
+                      kernel_of(s), 0);
   }
   if (pass == 0) return cudaSuccess;
   Offs<T, 5> q5;
@@ -335,66 +391,23 @@ __global__ void k_pack(const T *__restrict__ src, const int64_t *__restrict__ id
 // (n elements of (Np, 5, 3)): elements idx[0..n) (pack), or `first` and on.
 template <typename T>
 __global__ void k_grad_elems(bool pack, T *__restrict__ gq, const int64_t *__restrict__ idx, int64_t first, int64_t n,
-                             int64_t Np, int64_t nall, T *__restrict__ buf) {
+                             int64_t nall, T *__restrict__ buf, DensityOf<T> rho) {
+  const int64_t Np = (int64_t)rho.Nq * rho.Nq * rho.Nq;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < 15 * Np * n; t += (int64_t)gridDim.x * blockDim.x) {
     const int64_t i = t / (15 * Np);
     const int c = (int)(t / Np % 15);
-    T *r = grad_at(gq, Np, nall, idx ? idx[i] : first + i, t % Np, c % 5, c / 5);
-    if (pack) buf[t] = *r;
-    else *r = buf[t];
+    const int64_t el = idx ? idx[i] : first + i;
+    if (pack) buf[t] = grad_value(gq, Np, nall, el, t % Np, c % 5, c / 5, rho);
+    else *grad_at(gq, Np, nall, el, t % Np, c % 5, c / 5) = buf[t];
   }
 }
 cudaError_t grad_elems(cb_solver *s, bool pack, const int64_t *idx, int64_t first, int64_t n, void *buf) {
   const int64_t Np = nodes(s), nall = s->nelem + s->nghost;
   const unsigned grid = blocks_for(15 * Np * n);
   if (s->prec == 64)
-    k_grad_elems<double><<<grid, 256, 0, s->stream>>>(pack, (double *)s->gradQ, idx, first, n, Np, nall, (double *)buf);
+    k_grad_elems<double><<<grid, 256, 0, s->stream>>>(pack, (double *)s->gradQ, idx, first, n, nall, (double *)buf, density_of<double>(s));
   else
-    k_grad_elems<float><<<grid, 256, 0, s->stream>>>(pack, (float *)s->gradQ, idx, first, n, Np, nall, (float *)buf);
-  return cudaGetLastError();
-}
-
-// After an odd number of steps of a run whose gradient is kept as records: the
-// state goes back from the twin into Q, and the density of Q, which the last
-// stage read, into the twin (see rho_src).  One pass over memory: eight loads in
-// flight and one division per thread (with a division per value 10 us more on 35 MB).
-constexpr int COPY_BACK = 8;
-template <typename T, typename I>
-__global__ void __launch_bounds__(256) k_copy_back(T *__restrict__ Q, T *__restrict__ twin, uint32_t Np, uint32_t inv,
-                                                   int64_t total) {
-  const int64_t t0 = blockIdx.x * (int64_t)(256 * COPY_BACK);
-  const uint32_t r0 = (uint32_t)((I)t0 % (5 * Np)), w = 5 * Np;
-  // (inv = 2^32 / w rounded up: exact quotients for r < w + 2048 <= 8703)
-  auto density = [&](uint32_t d) {
-    const uint32_t r = r0 + d, m = r - __umulhi(r, inv) * w;
-    return m >= 3 * Np && m < 4 * Np;
-  };
-  T v[COPY_BACK], rho[COPY_BACK];
-#pragma unroll
-  for (int k = 0; k < COPY_BACK; ++k) {
-    const uint32_t d = threadIdx.x + 256 * k;
-    if (t0 + d < total) {
-      v[k] = twin[t0 + d];
-      if (density(d)) rho[k] = Q[t0 + d];
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < COPY_BACK; ++k) {
-    const uint32_t d = threadIdx.x + 256 * k;
-    if (t0 + d < total) {
-      if (density(d)) twin[t0 + d] = rho[k];
-      Q[t0 + d] = v[k];
-    }
-  }
-}
-template <typename T>
-cudaError_t copy_back(cb_solver *s) {
-  const int64_t Np = nodes(s), total = Np * 5 * s->nelem;
-  const unsigned grid = (unsigned)((total + 256 * COPY_BACK - 1) / (256 * COPY_BACK));
-  const uint32_t inv = (uint32_t)(((uint64_t)1 << 32) / (uint64_t)(5 * Np)) + 1;
-  T *Q = (T *)s->Q, *twin = (T *)s->Qalt;
-  if (total <= 0xffffffffll) k_copy_back<T, uint32_t><<<grid, 256, 0, s->stream>>>(Q, twin, (uint32_t)Np, inv, total);
-  else k_copy_back<T, int64_t><<<grid, 256, 0, s->stream>>>(Q, twin, (uint32_t)Np, inv, total);
+    k_grad_elems<float><<<grid, 256, 0, s->stream>>>(pack, (float *)s->gradQ, idx, first, n, nall, (float *)buf, density_of<float>(s));
   return cudaGetLastError();
 }
 
@@ -408,7 +421,7 @@ cudaError_t copy_back(cb_solver *s) {
 // raises ST_MESH.
 template <int DIM, typename T>
 __global__ void k_faces(bool pack, bool rec, T *__restrict__ arr, const int64_t *__restrict__ codes, int64_t n, int Nq,
-                        int W, int64_t nown, int64_t nghost, T *__restrict__ buf, unsigned *status) {
+                        int W, int64_t nown, int64_t nghost, T *__restrict__ buf, unsigned *status, DensityOf<T> rho) {
   const int Nfp = DIM == 2 ? Nq : Nq * Nq, Np = Nfp * Nq;
   const int64_t per = (int64_t)W * Nfp;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n * per; t += (int64_t)gridDim.x * blockDim.x) {
@@ -422,6 +435,10 @@ __global__ void k_faces(bool pack, bool rec, T *__restrict__ arr, const int64_t 
     }
     const int64_t el = pack ? e : nown + e;
     const int64_t node = face_node_rt<DIM>(Nq, f, fn);
+    if (rec && pack) {
+      buf[t] = grad_value(arr, Np, nown + nghost, el, node, c % 5, c / 5, rho);
+      continue;
+    }
     T *a = rec ? grad_at(arr, Np, nown + nghost, el, node, c % 5, c / 5) : arr + node + (int64_t)Np * (c + (int64_t)W * el);
     if (pack) buf[t] = *a;
     else *a = buf[t];
@@ -434,14 +451,14 @@ cudaError_t launch_faces(cb_solver *s, bool pack, int what, const int64_t *codes
   const int W = (s->dim == 2 ? 4 : 5) * (what ? s->dim : 1);
   T *arr = (T *)(what ? s->gradQ : (s->cur ? s->Qalt : s->Q));
   const bool rec = what && records(s);
-  const cudaError_t e = what ? complete_gradient(s) : pack ? cudaSuccess : complete_gradient(s, arr);
-  if (e != cudaSuccess) return e;
   const int64_t total = n * W * Nfp;
   const int grid = (int)std::min<int64_t>((total + 255) / 256, 148 * 16);
   if (s->dim == 2)
-    k_faces<2, T><<<grid, 256, 0, s->stream>>>(pack, rec, arr, codes, n, Nq, W, s->nelem, s->nghost, (T *)buf, s->status);
+    k_faces<2, T><<<grid, 256, 0, s->stream>>>(pack, rec, arr, codes, n, Nq, W, s->nelem, s->nghost, (T *)buf, s->status,
+                                               density_of<T>(s));
   else
-    k_faces<3, T><<<grid, 256, 0, s->stream>>>(pack, rec, arr, codes, n, Nq, W, s->nelem, s->nghost, (T *)buf, s->status);
+    k_faces<3, T><<<grid, 256, 0, s->stream>>>(pack, rec, arr, codes, n, Nq, W, s->nelem, s->nghost, (T *)buf, s->status,
+                                               density_of<T>(s));
   return cudaGetLastError();
 }
 
@@ -571,10 +588,10 @@ int cb_solver_pack(cb_solver *s, int what, const int64_t *elems, int64_t n, void
   if (!s || n < 0 || (n && (!elems || !buf)) || what < 0 || what > 1 || (what == 1 && !s->gradQ))
     return solver_fail(CB_ERR_ARG, "cb_solver_pack: bad arguments");
   if (!n) return CB_OK;
-  cudaError_t e = what ? complete_gradient(s) : cudaSuccess;
-  if (e == cudaSuccess && what && records(s)) {
+  cudaError_t e;
+  if (what && records(s)) {
     e = grad_elems(s, true, elems, 0, n, buf);
-  } else if (e == cudaSuccess) {
+  } else {
     const int64_t ew = nodes(s) * (s->dim == 2 ? 4 : 5) * (what ? s->dim : 1);
     const unsigned grid = blocks_for(n * ew);
     const void *src = what ? s->gradQ : (s->cur ? s->Qalt : s->Q);
@@ -599,8 +616,7 @@ int cb_solver_unpack(cb_solver *s, int what, const void *buf, int64_t first, int
   } else {
     const size_t ew = state_bytes(s) / (size_t)s->nelem * (what ? s->dim : 1);
     char *dst = (char *)(what ? s->gradQ : (s->cur ? s->Qalt : s->Q)) + ew * (size_t)(s->nelem + first);
-    if ((e = what ? cudaSuccess : complete_gradient(s, s->cur ? s->Qalt : s->Q)) == cudaSuccess)
-      e = cudaMemcpyAsync(dst, buf, ew * (size_t)n, cudaMemcpyDeviceToDevice, s->stream);
+    e = cudaMemcpyAsync(dst, buf, ew * (size_t)n, cudaMemcpyDeviceToDevice, s->stream);
   }
   return e == cudaSuccess ? CB_OK : solver_fail(CB_ERR_CUDA, "cb_solver_unpack: %s", cudaGetErrorString(e));
 }
@@ -663,6 +679,8 @@ int solver_create(cb_solver **out, int dim, int N, int precision, int64_t nelem,
     const size_t gbytes = w * (size_t)Np * ns * dim * (nelem + nghost);
     if ((e = cudaMalloc(&s->gradQ, gbytes)) != cudaSuccess) return bail(CB_ERR_NOMEM, "gradQ");
     cudaMemsetAsync(s->gradQ, 0, gbytes, s->stream);
+    if (dim == 3 && (e = cudaMalloc(&s->rho, w * (size_t)Np * (nelem + nghost))) != cudaSuccess)
+      return bail(CB_ERR_NOMEM, "density");
   }
   if (pingpong(s)) {
     if ((e = cudaMalloc(&s->Qalt, w * (size_t)Np * ns * (nelem + nghost))) != cudaSuccess)
@@ -704,7 +722,8 @@ int solver_create(cb_solver **out, int dim, int N, int precision, int64_t nelem,
     s->unfused = true;
     cudaFree(s->Qalt);
     cudaFree(s->nbr);
-    s->Qalt = nullptr;
+    cudaFree(s->rho);
+    s->Qalt = s->rho = nullptr;
     s->nbr = nullptr;
     h = 0;
     const size_t gbytes = w * (size_t)Np * ns * dim * nelem;
@@ -736,7 +755,6 @@ int cb_lsrk_run(cb_solver *s, int64_t nsteps, double dt) {
   if (e0 != cudaSuccess) return solver_fail(CB_ERR_CUDA, "gradient form: %s", cudaGetErrorString(e0));
   e0 = settle(s);  // a state left in the twin by the stage API
   if (e0 != cudaSuccess) return solver_fail(CB_ERR_CUDA, "state copy: %s", cudaGetErrorString(e0));
-  const bool rec = records_wanted(s);
   const int64_t per_graph = pingpong(s) ? 2 : 1;
   const int64_t reps = nsteps / per_graph, rem = nsteps % per_graph;
   cudaError_t e;
@@ -753,15 +771,9 @@ int cb_lsrk_run(cb_solver *s, int64_t nsteps, double dt) {
     if ((e = enqueue(s, dt, true, false)) != cudaSuccess)
       return solver_fail(CB_ERR_CUDA, "step launch: %s", cudaGetErrorString(e));
   }
-  // records: the density gradient is left to whoever packs it; the last stage's
-  // input (its density, where the state goes back from the twin into Q) stays in
-  // the twin until then
-  if (rec && s->nghost && (e = density_gradient(s, rem ? s->Q : s->Qalt)) != cudaSuccess)
-    return solver_fail(CB_ERR_CUDA, "density gradient: %s", cudaGetErrorString(e));
-  if (rec && !s->nghost) s->rho_src = s->Qalt;
-  if (rem && s->rho_src) e = s->prec == 64 ? copy_back<double>(s) : copy_back<float>(s);
-  else if (rem) e = cudaMemcpyAsync(s->Q, s->Qalt, state_bytes(s), cudaMemcpyDeviceToDevice, s->stream);
-  if (rem && e != cudaSuccess) return solver_fail(CB_ERR_CUDA, "state copy: %s", cudaGetErrorString(e));
+  if (records_wanted(s)) s->rho_live = true;
+  if (rem && (e = cudaMemcpyAsync(s->Q, s->Qalt, state_bytes(s), cudaMemcpyDeviceToDevice, s->stream)) != cudaSuccess)
+    return solver_fail(CB_ERR_CUDA, "state copy: %s", cudaGetErrorString(e));
   return CB_OK;
 }
 
@@ -811,8 +823,6 @@ int cb_solver_set_offset(cb_solver *s, const double *qref) {
         return solver_fail(CB_ERR_UNSUPPORTED, "state offsets: the viscous form of this order has none");
     return CB_OK;
   }
-  const cudaError_t e = complete_gradient(s);  // (of the state with its old offset)
-  if (e != cudaSuccess) return solver_fail(CB_ERR_CUDA, "cb_solver_set_offset: %s", cudaGetErrorString(e));
   for (int k = 0; k < (s->dim == 2 ? 4 : 5); ++k) s->qref[k] = qref[k];
   drop_graph(s);
   return CB_OK;
@@ -895,6 +905,7 @@ int cb_solver_destroy(cb_solver *s) {
   cudaFree(s->nbr);
   cudaFree(s->gradQ);
   cudaFree(s->rhs_gradQ);
+  cudaFree(s->rho);
   cudaFree(s->owned_geo);
   cudaFree(s->status);
   cudaFree(s->part);

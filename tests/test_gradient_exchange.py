@@ -243,3 +243,30 @@ def test_ghost_gradients_outlive_a_kernel_choice(before, after):
         for part in parts:
             part.close()
     assert max(relerr_fields(out[0], out[1])) < 1e-12
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+@pytest.mark.parametrize("kernel", [5, 1])
+@pytest.mark.parametrize("stages", [0, 1])
+def test_gradient_is_of_the_state_its_pass_read(stages, kernel, precision):
+    """What a caller writes over the current state after the gradient pass (in Q, or
+    in the twin after an odd number of stages) does not reach a packed gradient."""
+    import torch
+    m, Q, dt, phys = box(3, (3, 2, 3))
+    _, ref = plain_run(m, Q, dt, 0, phys, stages=stages + 1)
+    real = torch.float64 if precision == 64 else torch.float32
+    s = solver(m, Q, precision, phys, kernel)
+    for st in range(stages):
+        stage_pass(s, st, dt, 0)
+        stage_pass(s, st, dt, 1)
+    stage_pass(s, stages, dt, 0)
+    torch.cuda.synchronize()
+    if stages == 0:
+        s.Q.mul_(2.0).add_(1.0)
+    else:  # (unpack, what = 0, needs ghosts: an even stage call overwrites the buffer instead)
+        stage_pass(s, stages, dt, 1)
+        stage_pass(s, stages + 1, dt, 1)
+    torch.cuda.synchronize()
+    got = packed(s, m, np.arange(m.nelem), real)
+    assert gradient_error(got, ref) < (1e-10 if precision == 64 else 3e-4)
+    s.close()
