@@ -289,6 +289,32 @@ __device__ __forceinline__ void contract(const T *sF, const T *Ds, int el,
   }
 }
 
+// The same in 3-D in the order in which a grid line is summed by a march through its
+// planes (k_march_volume): ζ terms up to the node's own plane, the buoyancy before that
+// plane's, then the ξ and η terms, summed by themselves, then the planes above.
+template <int Nq, int EPB, typename T>
+__device__ __forceinline__ void contract_planes(const T *sF, const T *Ds, int el, int n, T rhoMJ, T grav, T *R) {
+  constexpr int NS = Lay<3>::NS, Np = ipow(Nq, 3), SP = EPB * Np;
+  const int i = n % Nq, j = (n / Nq) % Nq, k = n / (Nq * Nq);
+  const T *base = sF + el * Np;
+#pragma unroll
+  for (int s = 0; s < NS; ++s) {
+    const T *F = base + (0 * NS + s) * SP, *G = base + (1 * NS + s) * SP, *H = base + (2 * NS + s) * SP;
+    T t = T(0), acc = R[s];
+#pragma unroll
+    for (int m = 0; m < Nq; ++m) t += Ds[m + Nq * i] * F[m + Nq * (j + Nq * k)];
+#pragma unroll
+    for (int m = 0; m < Nq; ++m) t += Ds[m + Nq * j] * G[i + Nq * (m + Nq * k)];
+#pragma unroll
+    for (int m = 0; m < Nq; ++m) {
+      if (s == 2 && m == k) acc -= rhoMJ * grav;
+      acc += Ds[m + Nq * k] * H[i + Nq * (j + Nq * m)];
+      if (m == k) acc += t;
+    }
+    R[s] = acc;
+  }
+}
+
 // Same contraction with a sign (for the LDG passes, which subtract).
 template <int DIM, int Nq, int EPB, typename T>
 __device__ __forceinline__ void contract_sub(const T *sF, const T *Ds, int el,

@@ -37,13 +37,16 @@ k_volumerhs(T *__restrict__ rhs, const T *__restrict__ Q,
             const T *__restrict__ vgeo, const T *__restrict__ D, int64_t nelem,
             PhysT<T> p) {
   using C = Cfg<DIM, Nq>;
-  constexpr int NS = Lay<DIM>::NS, NVG = Lay<DIM>::NVG, Np = C::Np;
+  constexpr int NS = Lay<DIM>::NS, NVG = Lay<DIM>::NVG, Np = C::Np, IR = Lay<DIM>::IR;
+  // where large meshes run the march, its order of summation: a result does not
+  // depend on how many elements a call has
+  constexpr bool PLANES = DIM == 3 && march_volume_built(Nq, sizeof(T));
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T *Ds = reinterpret_cast<T *>(smem_raw);
   T *sF = Ds + Nq * Nq;
   load_D(Ds, D, Nq * Nq);
   const int64_t e0 = (int64_t)blockIdx.x * C::EPB;
-  T R[C::NPT][NS];
+  T R[C::NPT][NS], rhoMJ[PLANES ? C::NPT : 1];
 #pragma unroll
   for (int u = 0; u < C::NPT; ++u) {
     const int slot = threadIdx.x + u * C::THREADS;
@@ -59,7 +62,13 @@ k_volumerhs(T *__restrict__ rhs, const T *__restrict__ Q,
       T met[DIM][DIM], MJ;
       const T *vg = vgeo + (int64_t)Np * NVG * e;
       load_metric<DIM, T>(vg, n, Np, met, MJ);
-      pointwise_euler<DIM, Nq, C::EPB, T>(q, met, MJ, vg, n, el, sF, p, R[u]);
+      if constexpr (PLANES) {
+        T unused[NS] = {};
+        pointwise_euler<DIM, Nq, C::EPB, T>(q, met, MJ, vg, n, el, sF, p, unused);
+        rhoMJ[u] = MJ * q[IR];
+      } else {
+        pointwise_euler<DIM, Nq, C::EPB, T>(q, met, MJ, vg, n, el, sF, p, R[u]);
+      }
     }
   }
   __syncthreads();
@@ -69,7 +78,8 @@ k_volumerhs(T *__restrict__ rhs, const T *__restrict__ Q,
     const int el = slot / Np, n = slot % Np;
     const int64_t e = e0 + el;
     if (slot < C::SLOTS && e < nelem) {
-      contract<DIM, Nq, C::EPB, T>(sF, Ds, el, n, R[u]);
+      if constexpr (PLANES) contract_planes<Nq, C::EPB, T>(sF, Ds, el, n, rhoMJ[u], p.grav, R[u]);
+      else contract<DIM, Nq, C::EPB, T>(sF, Ds, el, n, R[u]);
 #pragma unroll
       for (int s = 0; s < NS; ++s) rhs[n + Np * (s + NS * e)] = R[u][s];
     }

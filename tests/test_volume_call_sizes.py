@@ -37,3 +37,31 @@ def test_volume_integral(N, n, precision):
     dg.volumerhs(3, N, d["r"], d["Q"], d["vgeo"], d["D"], m.nelem, dg.make_phys(**phys))
     out = dg.from_device(d["r"], h["Q"].shape).astype(np.float64)
     assert max(relerr_fields(out, w["r"])) < (1e-13 if precision == 64 else 1e-5)
+
+
+# elements on both sides of the block count from which the march runs
+@pytest.mark.parametrize("precision", [64, 32])
+@pytest.mark.parametrize("gravity", [0.0, 0.02])
+@pytest.mark.parametrize("N,few,many", [(2, 33, 7000), (3, 33, 4500), (4, 301, 2900), (5, 101, 1500), (6, 51, 700),
+                                        (7, 37, 700), (8, 31, 400), (9, 21, 300), (10, 17, 300)])
+def test_an_element_does_not_depend_on_the_count(N, few, many, gravity, precision):
+    """Bit for bit: the first elements of a large call against a call for them alone."""
+    import torch
+    real = torch.float64 if precision == 64 else torch.float32
+    g = torch.Generator(device="cuda").manual_seed(N)
+    Np = (N + 1) ** 3
+    def rand(*shape):
+        return torch.rand(*shape, generator=g, device="cuda", dtype=torch.float64)
+    Q = rand(many, 5, Np) - 0.5
+    Q[:, 3] += 1.5  # density and total energy: positive pressure
+    Q[:, 4] += 4.0
+    Q, vgeo, D, r = (t.to(real).reshape(-1).contiguous() for t in
+                     (Q, rand(many, 14, Np) + 0.1, rand(N + 1, N + 1) - 0.5, rand(many, 5, Np) - 0.5))
+    a, b = r.clone(), r.clone()
+    ph = dg.make_phys(**dict(dg.WORKLOAD_PHYS, gravity=gravity))
+    dg.volumerhs(3, N, a, Q, vgeo, D, many, ph)
+    dg.volumerhs(3, N, b, Q, vgeo, D, few, ph)
+    k = few * 5 * Np
+    assert torch.isfinite(a).all()
+    assert torch.equal(a[:k], b[:k])
+    assert torch.equal(b[k:], r[k:])
