@@ -1004,12 +1004,18 @@ struct Launch {
   // Whether a chained launch of a persistent kernel of `grid` blocks is
   // programmatic.  What overlaps is its prologue; what it costs is the even spread
   // of the blocks: they start wherever an SM has room, so that blocks with a group
-  // more than the others meet on one SM.  Worth it where every block has one group or
-  // the prologue zeroes padded flux rows (2-D, us a step plain / programmatic: FP64
-  // N=4 60^2 42.1 / 39.0, FP32 N=5 72^2 42.1 / 39.2; unpadded with 1.35 groups a block,
-  // N=7 40^2 34.9 / 38.0; 3-D N=7 FP32 24^3 1118 / 1186, N=3 FP64 40^3 1555 / 1640).
+  // more than the others meet on one SM.  Worth it where few or nearly all blocks of a wave
+  // have a group more, or the prologue zeroes padded flux rows (us a step plain /
+  // programmatic, groups a block in brackets.  Unpadded: 2-D FP64 N=3 72^2 36.3 / 33.8
+  // (1.1), 3-D FP64 N=5 7^3 42.9 / 41.0 (1.2); 2-D N=7 FP64 40^2 35.9 / 37.9 (1.35), FP32 60^2
+  // 35.9 / 38.9 (1.5); 3-D FP64 N=5 8^3 49.2 / 47.2 (1.7), 2-D FP64 N=3 100^2 50.4 / 48.2
+  // (2.1), FP32 N=7 72^2 48.1 / 45.2 (2.2); 3-D FP64 N=7 9^3 128.1 / 130.3 (2.5), N=3 17^3
+  // 141 / 152 (4.2), 2-D FP64 N=5 130^2 139 / 144 (8.2).  Padded: 2-D FP32 N=5 85^2 55.4 / 46.5
+  // (1.7), 200^2 203 / 189 (9.7)).
   static constexpr bool PADDED = Pipe2<DIM, Nq, T>::MV > Nq;
-  static int chain_pays(int chained, int64_t groups, int64_t grid) { return chained && (PADDED || groups <= grid); }
+  static int chain_pays(int chained, int64_t groups, int64_t grid) {
+    return chained && (PADDED || 4 * groups <= 5 * grid || (10 * groups >= 16 * grid && 10 * groups <= 22 * grid));
+  }
   // The stage kernel that choice 0 resolves to on a mesh of nelem elements.
   static int choice(int64_t nelem, bool gravity) {
     if (MARCH) return nelem <= num_sms() ? 3 : 5;
